@@ -130,21 +130,34 @@ SPH_HD double ln_pos(double x)
     return dadd(dmul((double) e, 0.6931471805599453), dmul(2.0, sum));
 }
 
+// On the device the lanes of a warp meet again here after a rejection loop (particle() is called by
+// whole warps): code behind it would otherwise run once for each try at which some lane left the loop.
+SPH_HD void lanes_meet()
+{
+#ifdef __CUDA_ARCH__
+    __syncwarp();
+#endif
+}
+
 // two independent standard normals
 SPH_HD void polar_pair(uint64_t &s, double &g0, double &g1)
 {
-    for (int t = 0; t < 64; t++) {
-        const double u = sym(s), v = sym(s);
-        const double q = dadd(dmul(u, u), dmul(v, v));
-        if (q > 0.0 && q < 1.0) {
-            const double f = dsqrt(ddiv(dmul(-2.0, ln_pos(q)), q));
-            g0 = dmul(u, f);
-            g1 = dmul(v, f);
-            return;
+    double u = 0.0, v = 0.0, q = 1.0;
+    bool found = false;
+    for (int t = 0; t < 64 && !found; t++) {
+        const double a = sym(s), b = sym(s);
+        const double r = dadd(dmul(a, a), dmul(b, b));
+        found = r > 0.0 && r < 1.0;
+        if (found) {
+            u = a;
+            v = b;
+            q = r;
         }
     }
-    g0 = 0.0;
-    g1 = 0.0;
+    lanes_meet();
+    const double f = dsqrt(ddiv(dmul(-2.0, ln_pos(q)), q));
+    g0 = found ? dmul(u, f) : 0.0;
+    g1 = found ? dmul(v, f) : 0.0;
 }
 
 // particle k of emission step `step`: position on the disc of `radius` around `center` in the
@@ -163,6 +176,7 @@ SPH_HD void particle(uint64_t seed, uint32_t step, uint32_t k, const float cente
             break;
         }
     }
+    lanes_meet();
     xyz[0] = to_float(dadd((double) center[0], dmul((double) radius, dx)));
     xyz[1] = center[1];
     xyz[2] = to_float(dadd((double) center[2], dmul((double) radius, dz)));
