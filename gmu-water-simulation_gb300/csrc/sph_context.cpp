@@ -67,6 +67,7 @@ struct sph_ctx {
     uint32_t graph_n = 0;
     std::vector<uint32_t> scene_off_host;
     Tune tune;
+    int dense_mode = 3;        // force variant that the last density pass prepared for
     bool tune_pinned = false;  // variants set explicitly: the cache does not override them
     bool cell_pinned = false;  // cell multiple set explicitly: the autotuner keeps it
     // front-end handoff (allocated by the first handoff or export)
@@ -479,7 +480,19 @@ int run_density(sph_ctx *c)
         CK(c, mixed_density(c->b, c->n, make_consts<float>(c, c->tune.cell_mult), make_mix(c->prm),
                             c->tune.cell_mult, c->stream));
     else CK(c, Launch<R>::density(c->b, c->n, make_consts<R>(c, c->tune.cell_mult), c->tune, c->stream));
+    c->dense_mode = c->tune.forces_mode;
     return SPH_OK;
+}
+
+// The variant set now, or, where it was changed since the density pass to one that reads the force
+// records and that pass wrote none (4 to 6: masks alone), a variant that needs only the masks. All
+// of them give the same bits.
+Tune forces_tune(const sph_ctx *c)
+{
+    Tune t = c->tune;
+    const bool reads_records = t.forces_mode == 3 || (t.forces_mode >= 7 && t.forces_mode <= 11);
+    if (reads_records && c->dense_mode >= 4 && c->dense_mode <= 6) t.forces_mode = c->dense_mode;
+    return t;
 }
 template <class R>
 int run_forces(sph_ctx *c)
@@ -488,7 +501,7 @@ int run_forces(sph_ctx *c)
     if (is_mixed(c))
         CK(c, mixed_forces(c->b, c->n, make_consts<float>(c, c->tune.cell_mult), make_mix(c->prm), rec,
                            c->tune.forces_mode, c->tune.cell_mult, c->stream));
-    else CK(c, Launch<R>::forces(c->b, c->n, make_consts<R>(c, c->tune.cell_mult), rec, c->tune, c->stream));
+    else CK(c, Launch<R>::forces(c->b, c->n, make_consts<R>(c, c->tune.cell_mult), rec, forces_tune(c), c->stream));
     return SPH_OK;
 }
 
@@ -817,6 +830,7 @@ int sph_debug_check(sph_ctx *c, uint32_t *flags)
     *flags = 0;
     CK(c, check_flags_kernels(flags));
     CK(c, check_flags_mixed(flags));
+    CK(c, check_flags_group(flags));
     CK(c, check_flags_handoff(flags));
     CK(c, check_flags_noalloc(flags));
     std::vector<unsigned char> buf(kCanaryBytes);

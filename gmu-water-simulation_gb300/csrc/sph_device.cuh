@@ -358,22 +358,32 @@ __device__ __forceinline__ void pair_force(const Vec4<R> &pi, const Vec4<R> &vi,
     pair_terms<R>(pi, vi, qi, pj, vj, qj, invj, c, fpx, fpy, fpz, fvx, fvy, fvz);
 }
 
+// The position difference d and the two factors of one pair's force terms: w * d is added to the
+// pressure sums, l times the velocity difference to the viscosity sums.
+template <class R>
+__device__ __forceinline__ void pair_factors(const Vec4<R> &pi, R qi, const Vec4<R> &pj, R qj, R invj,
+                                             const Consts<R> &c, R &dx, R &dy, R &dz, R &w, R &l)
+{
+    dx = rsub(pi.x, pj.x), dy = rsub(pi.y, pj.y), dz = rsub(pi.z, pj.z);
+    const R r2 = rfma(dz, dz, rfma(dy, dy, rmul(dx, dx)));
+    const R rinv = inv_sqrt(r2);
+    const R hr = rfma(-r2, rinv, c.h);
+    // (p_i/rho_i^2 + p_j/rho_j^2) grad W and lap W / rho_j, the constants carried by qi, qj, invj
+    w = rmul(radd(qi, qj), rmul(rmul(hr, hr), rinv));
+    l = rmul(hr, invj);
+}
+
 // The same terms from a neighbour's records already loaded (pair_force's arithmetic).
 template <class R>
 __device__ __forceinline__ void pair_terms(const Vec4<R> &pi, const Vec4<R> &vi, R qi, const Vec4<R> &pj,
                                            const Vec4<R> &vj, R qj, R invj, const Consts<R> &c, R &fpx, R &fpy,
                                            R &fpz, R &fvx, R &fvy, R &fvz)
 {
-    const R dx = rsub(pi.x, pj.x), dy = rsub(pi.y, pj.y), dz = rsub(pi.z, pj.z);
-    const R r2 = rfma(dz, dz, rfma(dy, dy, rmul(dx, dx)));
-    const R rinv = inv_sqrt(r2);
-    const R hr = rfma(-r2, rinv, c.h);
-    // (p_i/rho_i^2 + p_j/rho_j^2) grad W and lap W / rho_j, the constants carried by qi, qj, invj
-    const R w = rmul(radd(qi, qj), rmul(rmul(hr, hr), rinv));
+    R dx, dy, dz, w, l;
+    pair_factors<R>(pi, qi, pj, qj, invj, c, dx, dy, dz, w, l);
     fpx = rfma(w, dx, fpx);
     fpy = rfma(w, dy, fpy);
     fpz = rfma(w, dz, fpz);
-    const R l = rmul(hr, invj);
     fvx = rfma(rsub(vj.x, vi.x), l, fvx);
     fvy = rfma(rsub(vj.y, vi.y), l, fvy);
     fvz = rfma(rsub(vj.z, vi.z), l, fvz);

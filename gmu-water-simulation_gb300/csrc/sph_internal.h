@@ -123,8 +123,9 @@ struct MixConsts {
 //               with that many consecutive particles per thread
 //   forces_mode: 0 = pair terms inside the candidate loop; 1/2 = compacted neighbour list
 //               of 32/64 entries per thread in shared memory; 3..11 = driven by the neighbour
-//               masks that the density pass then writes (density_p is ignored): 3/4 one
-//               neighbour per iteration without/with a 64-register cap, 5/6 two per
+//               masks that the density pass then writes (density_p is ignored): 3, the default,
+//               in group form (sph_group.cu) for up to kGroupMax particles of the plain form, else
+//               as 4; 3/4 one neighbour per iteration without/with a 64-register cap, 5/6 two per
 //               iteration with/without it, 7 as 6 with each neighbour's terms read from one
 //               packed force record (two 16-byte loads from one 32-byte record), 8 and 9 as
 //               7 at 48 and 40 registers, 10 and 11 as 9 and 8 in blocks of 128 threads
@@ -226,8 +227,15 @@ cudaError_t ref_grid_build(const float *xyz, uint32_t n, int3 res, float3 half, 
 // checked builds: OR each translation unit's device check flags into *out and clear them
 cudaError_t check_flags_kernels(uint32_t *out);
 cudaError_t check_flags_mixed(uint32_t *out);
+cudaError_t check_flags_group(uint32_t *out);
 cudaError_t check_flags_handoff(uint32_t *out);
 cudaError_t check_flags_noalloc(uint32_t *out);
+
+// Group forms of the neighbour passes (sph_group.cu): several lanes a particle, for scenes too small to
+// fill the GPU with one thread each. The default variant (3) uses them for up to kGroupMax particles.
+constexpr uint32_t kGroupMax = 32768;
+cudaError_t group_density(const DevBufs &b, uint32_t n, Consts<float> c, cudaStream_t st);
+cudaError_t group_forces(const DevBufs &b, uint32_t n, Consts<float> c, bool record_acc, cudaStream_t st);
 
 // mixed-precision passes (sph_mixed.cu)
 cudaError_t mixed_permute(const DevBufs &b, uint32_t n, Consts<float> c, MixConsts mc, cudaStream_t st);

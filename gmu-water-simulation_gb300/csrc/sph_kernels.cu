@@ -981,6 +981,8 @@ cudaError_t Launch<R>::density(const DevBufs &b, uint32_t n, Consts<R> c, const 
         k_density_all<R><<<nblk(n, 256), 256, 0, st>>>(pos, aux, b.start, b.scenes, n, c);
         return cudaGetLastError();
     }
+    if constexpr (sizeof(R) == 4)
+        if (t.forces_mode == 3 && t.cell_mult == 1 && n <= kGroupMax) return group_density(b, n, c, st);
     if (t.forces_mode >= 7) {  // masks and force records
         if (t.cell_mult == 2) {
             if constexpr (sizeof(R) == 4)
@@ -1040,6 +1042,8 @@ cudaError_t Launch<R>::forces(const DevBufs &b, uint32_t n, Consts<R> c, bool re
             return cudaErrorInvalidValue;
         }
     }
+    if constexpr (sizeof(R) == 4)
+        if (t.forces_mode == 3 && n <= kGroupMax) return group_forces(b, n, c, record_acc, st);
     switch (t.forces_mode) {
     case Tune::ALL_PAIRS:
         k_forces_all<R><<<nblk(n, 256), 256, 0, st>>>(pos, vel, aux, b.start, b.scenes, b.obstacles, n, c, po, vo, ao,
