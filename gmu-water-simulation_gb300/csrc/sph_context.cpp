@@ -484,14 +484,15 @@ int run_density(sph_ctx *c)
     return SPH_OK;
 }
 
-// The variant set now, or, where it was changed since the density pass to one that reads the force
-// records and that pass wrote none (4 to 6: masks alone), a variant that needs only the masks. All
-// of them give the same bits.
+// The variant set now, or, where it was changed since the density pass to one that reads what that
+// pass did not write, the variant of that pass: the force records (plain, 4 to 6 write masks alone),
+// the masks (FP64, 3 writes none). All of them give the same bits.
 Tune forces_tune(const sph_ctx *c)
 {
     Tune t = c->tune;
-    const bool reads_records = t.forces_mode == 3 || (t.forces_mode >= 7 && t.forces_mode <= 11);
-    if (reads_records && c->dense_mode >= 4 && c->dense_mode <= 6) t.forces_mode = c->dense_mode;
+    const bool reads_records = (t.forces_mode == 3 && !is_f64(c)) || (t.forces_mode >= 7 && t.forces_mode <= 11);
+    if (is_f64(c) && c->dense_mode == 3 && t.forces_mode >= 4 && t.forces_mode <= 11) t.forces_mode = 3;
+    else if (reads_records && c->dense_mode >= 4 && c->dense_mode <= 6) t.forces_mode = c->dense_mode;
     return t;
 }
 template <class R>

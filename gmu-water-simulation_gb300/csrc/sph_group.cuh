@@ -50,6 +50,22 @@ struct Group {
     }
 };
 
+// The sums of a block's particles in shared memory, so that its first warp finishes them with one lane
+// each: the per-particle epilogue would otherwise run with one lane of every group.
+template <class R, int G>
+struct GroupSums {
+    R f[Group<G>::PER_BLOCK][6];  // pressure x, y, z, viscosity x, y, z
+    __device__ __forceinline__ void put(const Group<G> &g, R fp, R fv)
+    {
+        const int k = g.warp * Group<G>::PER_WARP + g.slot;
+        if (g.gl < 3) {
+            f[k][g.gl] = fp;
+            f[k][3 + g.gl] = fv;
+        }
+        __syncthreads();
+    }
+};
+
 // The nine rows (dy, dz) of three cells of size h around a particle, in the order of the other
 // forms: lane r % G of a group holds first candidate and length of row r (0 beyond the grid).
 template <int G>

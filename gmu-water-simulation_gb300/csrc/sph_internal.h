@@ -102,8 +102,18 @@ __host__ __device__ inline int cell_axis(float p, float half, float inv_h, doubl
     return (int) floor(q);
 }
 
+// The same for a double coordinate: rounding it to float first moves the quotient by at most
+// 2^-24 |p| / h more, so the margin carries the coordinate's own size beside the quotient's. (The exact
+// formula's FP64 division costs more than the rest of a particle's cell arithmetic.)
 __host__ __device__ inline int cell_axis(double p, float half, float inv_h, double h_d, int res)
 {
+    const float qf = ((float) p + half) * inv_h;
+    const float rq = rintf(qf);
+    if (fabsf(qf - rq) > (fabsf(qf) + half * inv_h + 1.0f) * 6.0e-7f) {
+        if (qf < 0.0f) return 0;
+        if (qf >= (float) res) return res - 1;
+        return (int) floorf(qf);
+    }
     const double q = (p + (double) half) / h_d;
     if (!(q >= 0.0)) return 0;
     if (q >= (double) res) return res - 1;
@@ -124,8 +134,8 @@ struct MixConsts {
 //   forces_mode: 0 = pair terms inside the candidate loop; 1/2 = compacted neighbour list
 //               of 32/64 entries per thread in shared memory; 3..11 = driven by the neighbour
 //               masks that the density pass then writes (density_p is ignored): 3, the default,
-//               in group form (sph_group.cu) for up to kGroupMax particles of the plain form, else
-//               as 4; 3/4 one neighbour per iteration without/with a 64-register cap, 5/6 two per
+//               in group form (sph_group.cu) for up to kGroupMax particles of the plain form and for
+//               the FP64 form, else as 4; 3/4 one neighbour per iteration without/with a 64-register cap, 5/6 two per
 //               iteration with/without it, 7 as 6 with each neighbour's terms read from one
 //               packed force record (two 16-byte loads from one 32-byte record), 8 and 9 as
 //               7 at 48 and 40 registers, 10 and 11 as 9 and 8 in blocks of 128 threads
@@ -232,10 +242,13 @@ cudaError_t check_flags_handoff(uint32_t *out);
 cudaError_t check_flags_noalloc(uint32_t *out);
 
 // Group forms of the neighbour passes (sph_group.cu): several lanes a particle, for scenes too small to
-// fill the GPU with one thread each. The default variant (3) uses them for up to kGroupMax particles.
+// fill the GPU with one thread each. The default variant (3) uses them for up to kGroupMax particles of
+// the plain form and for any number of the FP64 form (which needs no masks and no records there).
 constexpr uint32_t kGroupMax = 32768;
 cudaError_t group_density(const DevBufs &b, uint32_t n, Consts<float> c, cudaStream_t st);
 cudaError_t group_forces(const DevBufs &b, uint32_t n, Consts<float> c, bool record_acc, cudaStream_t st);
+cudaError_t group_density(const DevBufs &b, uint32_t n, Consts<double> c, cudaStream_t st);
+cudaError_t group_forces(const DevBufs &b, uint32_t n, Consts<double> c, bool record_acc, cudaStream_t st);
 
 // mixed-precision passes (sph_mixed.cu)
 cudaError_t mixed_permute(const DevBufs &b, uint32_t n, Consts<float> c, MixConsts mc, cudaStream_t st);

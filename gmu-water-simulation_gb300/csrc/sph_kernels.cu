@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(256) k_rank_permute(const uint2 *__restrict__ 
                                                       const Vec4<R> *__restrict__ pos_u,
                                                       const Vec4<R> *__restrict__ vel_u,
                                                       Vec4<R> *__restrict__ pos_s, Vec4<R> *__restrict__ vel_s,
-                                                      uint32_t *__restrict__ big)
+                                                      uint32_t *__restrict__ big, float *__restrict__ posf)
 {
     chain_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) big[0] = 0;  // the crowded-cell list is used: empty for the next scan
@@ -286,6 +286,11 @@ __global__ void __launch_bounds__(256) k_rank_permute(const uint2 *__restrict__ 
     if (!sph_check(dst < e, CHK_SORT)) return;
     st4(pos_s + dst, p);
     st4(vel_s + dst, v);
+    if constexpr (sizeof(R) == 8) {  // rounded positions for the FP64 form's first test of its candidates
+        posf[3 * (size_t) dst] = (float) p.x;
+        posf[3 * (size_t) dst + 1] = (float) p.y;
+        posf[3 * (size_t) dst + 2] = (float) p.z;
+    }
 }
 
 // ------------------------------------------------------------------------------------
@@ -959,7 +964,7 @@ cudaError_t Launch<R>::permute(const DevBufs &b, uint32_t n, uint32_t ncells, cu
     if (e != cudaSuccess) return e;
     return launch_chained(k_rank_permute<R>, nblk(n, 256), 256, st, b.cid_u, n, b.start, b.tmp,
                           (const Vec4<R> *) b.pos_u, (const Vec4<R> *) b.vel_u, (Vec4<R> *) b.pos_s,
-                          (Vec4<R> *) b.vel_s, b.big);
+                          (Vec4<R> *) b.vel_s, b.big, b.st_xyz);
 }
 
 template <class R>
@@ -981,8 +986,8 @@ cudaError_t Launch<R>::density(const DevBufs &b, uint32_t n, Consts<R> c, const 
         k_density_all<R><<<nblk(n, 256), 256, 0, st>>>(pos, aux, b.start, b.scenes, n, c);
         return cudaGetLastError();
     }
-    if constexpr (sizeof(R) == 4)
-        if (t.forces_mode == 3 && t.cell_mult == 1 && n <= kGroupMax) return group_density(b, n, c, st);
+    if (t.forces_mode == 3 && t.cell_mult == 1 && (sizeof(R) == 8 || n <= kGroupMax))
+        return group_density(b, n, c, st);
     if (t.forces_mode >= 7) {  // masks and force records
         if (t.cell_mult == 2) {
             if constexpr (sizeof(R) == 4)
@@ -1042,8 +1047,7 @@ cudaError_t Launch<R>::forces(const DevBufs &b, uint32_t n, Consts<R> c, bool re
             return cudaErrorInvalidValue;
         }
     }
-    if constexpr (sizeof(R) == 4)
-        if (t.forces_mode == 3 && n <= kGroupMax) return group_forces(b, n, c, record_acc, st);
+    if (t.forces_mode == 3 && (sizeof(R) == 8 || n <= kGroupMax)) return group_forces(b, n, c, record_acc, st);
     switch (t.forces_mode) {
     case Tune::ALL_PAIRS:
         k_forces_all<R><<<nblk(n, 256), 256, 0, st>>>(pos, vel, aux, b.start, b.scenes, b.obstacles, n, c, po, vo, ao,

@@ -49,6 +49,37 @@ def test_plain_group_form_equals_one_thread_forms(sphlib, n, kind):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,kind", [(1, "lattice"), (35, "clump"), (1501, "clump"), (16383, "lattice"),
+                                    (16384, "lattice"), (16385, "lattice")])
+def test_f64_group_form_equals_one_thread_forms(sphlib, n, kind):
+    """Also pairs close to r = h, where the float test passes them on to the exact one: the clump's
+    many pairs, and a pair of particles moved to within a few float ulps of h."""
+    box, pos, vel = scene(n, kind, 2)
+    if n > 2:
+        pos[1] = pos[0] + np.array([0.0457, 0, 0], np.float32)
+        pos[2] = np.nextafter(pos[1], np.float32(-1), dtype=np.float32)
+    got = run(sphlib, box, pos, vel, None, sphlib.SPH_F64)
+    for variant in (0, 4):
+        ref = run(sphlib, box, pos, vel, variant, sphlib.SPH_F64)
+        for k in ref:
+            assert np.array_equal(got[k], ref[k]), (n, kind, variant, k)
+
+
+@pytest.mark.gpu
+def test_f64_far_coordinates(sphlib):
+    """Coordinates whose float rounding is larger than h, beyond the float range of squares, and
+    infinite: the float test decides nothing there and the exact one gives the mask form's bits."""
+    box, pos, vel = scene(300, "clump", 3)
+    pos[:20] = np.float32(3.0e7) + np.arange(60, dtype=np.float32).reshape(20, 3)
+    pos[20:24] = np.float32(2.5e30)
+    pos[24, 1] = np.inf
+    got = run(sphlib, box, pos, vel, None, sphlib.SPH_F64, steps=2)
+    ref = run(sphlib, box, pos, vel, 4, sphlib.SPH_F64, steps=2)
+    for k in ref:
+        assert np.array_equal(got[k], ref[k], equal_nan=True), k
+
+
+@pytest.mark.gpu
 def test_variant_changed_between_the_passes(sphlib):
     """A density pass that wrote masks and no records (variants 4 to 6) is followed by a force pass of
     any mask-driven variant: the same bits."""
@@ -56,6 +87,26 @@ def test_variant_changed_between_the_passes(sphlib):
     ref = run(sphlib, box, pos, vel, 4, steps=1)
     for dense, forces in ((4, 3), (6, 3), (5, 10), (3, 4), (3, 7), (10, 3)):
         ctx = sphlib.SphContext(box, pos.shape[0], gravity=G981, flags=sphlib.SPH_FLAG_RECORD_ACC)
+        ctx.upload(pos, vel)
+        ctx.set_variant(0, dense)
+        ctx.pass_grid()
+        ctx.pass_density()
+        ctx.set_variant(0, forces)
+        ctx.pass_forces()
+        got = ctx.download(acc=True)
+        ctx.close()
+        for k in ref:
+            assert np.array_equal(got[k], ref[k]), (dense, forces, k)
+
+
+@pytest.mark.gpu
+def test_f64_variant_changed_between_the_passes(sphlib):
+    """The FP64 density pass of variant 3 writes neither masks nor records."""
+    box, pos, vel = scene(2003, "lattice", 5)
+    ref = run(sphlib, box, pos, vel, 4, sphlib.SPH_F64, steps=1)
+    for dense, forces in ((3, 4), (3, 10), (4, 3), (4, 9), (10, 3)):
+        ctx = sphlib.SphContext(box, pos.shape[0], gravity=G981, flags=sphlib.SPH_FLAG_RECORD_ACC,
+                                precision=sphlib.SPH_F64)
         ctx.upload(pos, vel)
         ctx.set_variant(0, dense)
         ctx.pass_grid()
