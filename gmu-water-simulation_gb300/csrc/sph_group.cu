@@ -10,9 +10,6 @@
 namespace sph {
 
 // ---- plain FP32 ------------------------------------------------------------------------------
-constexpr int kListFlush = 96;              // entries from which a list is worked off ...
-constexpr int kListLen = kListFlush + 32 + 8;  // ... before the next 32 candidates (+8: other banks per group)
-
 // Bound by the latency of a particle's walk (20 cycles an instruction at one warp a scheduler): 18.4 us
 // with one thread a particle, 14.3 us with 8 or 16 lanes, for 8,000 particles at rest; fallen 28.7 and
 // 14.3 us. Writes what the mask form writes: the words of accepted candidates and the force records.
@@ -78,25 +75,6 @@ __global__ void __launch_bounds__(kGroupThreads) k_density_group(
     const Vec4<float> vi = ld4(vel + i);
     st4(frec + 2 * (size_t) i, Vec4<float>{pi.x, pi.y, pi.z, ar.z});
     st4(frec + 2 * (size_t) i + 1, Vec4<float>{vi.x, vi.y, vi.z, ar.w});
-}
-
-// One neighbour's factors and differences, waiting for the ordered sums: (difference of positions,
-// difference of velocities) per axis, then the two factors.
-template <class R>
-struct alignas(8 * sizeof(R)) PairOut {
-    R v[8];
-};
-
-// Sums of one axis each in lanes 0 to 2 of a group: fp += w * d, fv += dv * l over cnt pairs in order.
-template <class R>
-__device__ __forceinline__ void add_pairs(const PairOut<R> *out, uint32_t cnt, unsigned axis, R &fp, R &fv)
-{
-#pragma unroll 4
-    for (uint32_t s = 0; s < cnt; s++) {
-        const R d = out[s].v[2 * axis], dv = out[s].v[2 * axis + 1];
-        fp = rfma(out[s].v[6], d, fp);
-        fv = rfma(dv, out[s].v[7], fv);
-    }
 }
 
 // The accepted neighbours (from the density pass's words) are listed in order, the factors of G or 16
@@ -413,8 +391,6 @@ static cudaError_t forces_g(const DevBufs &b, uint32_t n, Consts<float> c, bool 
 // lanes shorten a particle's serial walk, but the compaction makes the instructions per candidate
 // about 1.5 times as many, which is what counts once the warps fill the GPU. (4 lanes gain nothing
 // anywhere, and 32 only a few us below 2,000 particles.)
-constexpr uint32_t kGroupWide = 10240;
-
 cudaError_t group_density(const DevBufs &b, uint32_t n, Consts<float> c, cudaStream_t st)
 {
     return n <= kGroupWide ? density_g<16>(b, n, c, st) : density_g<8>(b, n, c, st);

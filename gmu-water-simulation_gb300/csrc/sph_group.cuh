@@ -104,4 +104,26 @@ struct GroupRows {
     }
 };
 
+constexpr int kListFlush = 96;              // entries from which a list is worked off ...
+constexpr int kListLen = kListFlush + 32 + 8;  // ... before the next 32 candidates (+8: other banks per group)
+
+// One neighbour's factors and differences, waiting for the ordered sums: (difference of positions,
+// difference of velocities) per axis, then the two factors.
+template <class R>
+struct alignas(8 * sizeof(R)) PairOut {
+    R v[8];
+};
+
+// Sums of one axis each in lanes 0 to 2 of a group: fp += w * d, fv += dv * l over cnt pairs in order.
+template <class R>
+__device__ __forceinline__ void add_pairs(const PairOut<R> *out, uint32_t cnt, unsigned axis, R &fp, R &fv)
+{
+#pragma unroll 4
+    for (uint32_t s = 0; s < cnt; s++) {
+        const R d = out[s].v[2 * axis], dv = out[s].v[2 * axis + 1];
+        fp = rfma(out[s].v[6], d, fp);
+        fv = rfma(dv, out[s].v[7], fv);
+    }
+}
+
 }  // namespace sph

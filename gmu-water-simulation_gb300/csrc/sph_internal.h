@@ -244,7 +244,7 @@ cudaError_t check_flags_noalloc(uint32_t *out);
 // Group forms of the neighbour passes (sph_group.cu): several lanes a particle, for scenes too small to
 // fill the GPU with one thread each. The default variant (3) uses them for up to kGroupMax particles of
 // the plain form and for any number of the FP64 form (which needs no masks and no records there).
-constexpr uint32_t kGroupMax = 32768;
+constexpr uint32_t kGroupWide = 10240, kGroupMax = 32768;
 cudaError_t group_density(const DevBufs &b, uint32_t n, Consts<float> c, cudaStream_t st);
 cudaError_t group_forces(const DevBufs &b, uint32_t n, Consts<float> c, bool record_acc, cudaStream_t st);
 cudaError_t group_density(const DevBufs &b, uint32_t n, Consts<double> c, cudaStream_t st);

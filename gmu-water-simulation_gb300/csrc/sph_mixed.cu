@@ -23,6 +23,7 @@
 #include <stdint.h>
 
 #include "sph_device.cuh"
+#include "sph_group.cuh"
 #include "sph_internal.h"
 
 namespace sph {
@@ -177,27 +178,68 @@ __global__ void __launch_bounds__(128) k_density_mixed(const Vec4<float> *__rest
 // ---- forces: mask-driven, code-unit displacements, one 16-byte record per neighbour ----------
 // Pressure and viscosity terms of one neighbour from its record (the plain form's pair terms in
 // code units; src/CCPUParticleSimulator.cpp:177-183). qs = own p/rho^2 * 2^10.
-__device__ __forceinline__ void mixed_pair(uint2 gi, const Vec4<float> &vi, float qs, uint4 r, const MixConsts &mc,
-                                           float &fpx, float &fpy, float &fpz, float &fvx, float &fvy, float &fvz)
+// mixed_factors: the difference d, the neighbour's velocity and the two factors; w * d and
+// l * (vj - vi) are summed.
+__device__ __forceinline__ void mixed_factors(uint2 gi, float qs, uint4 r, const MixConsts &mc, float &dx, float &dy,
+                                              float &dz, float &vjx, float &vjy, float &vjz, float &wgt, float &l)
 {
-    float dx, dy, dz;
     code_delta(gi, make_uint2(r.x, r.y), dx, dy, dz);
-    const float vjx = unpack_half2(r.y >> 16).x;
+    vjx = unpack_half2(r.y >> 16).x;
     const float2 vyz = unpack_half2(r.z);
     const float2 qv = unpack_half2(r.w);
+    vjy = vyz.x;
+    vjz = vyz.y;
     // at least one unit apart: two particles sharing a code (closer than the 5.6 um resolution)
     // get no pressure direction rather than a 0/0
     const float r2 = fmaxf(dx * dx + dy * dy + dz * dz, 1.0f);
     const float rinv = rsqrtf(r2);
     const float hr = QUNITS - r2 * rinv;
-    const float wgt = (qs + qv.x) * (mc.spiky_q * (1.0f / Q_SCALE) * hr * hr * rinv);
+    wgt = (qs + qv.x) * (mc.spiky_q * (1.0f / Q_SCALE) * hr * hr * rinv);
+    l = mc.visc_q * (1.0f / INV_SCALE) * hr * qv.y;
+}
+
+__device__ __forceinline__ void mixed_pair(uint2 gi, const Vec4<float> &vi, float qs, uint4 r, const MixConsts &mc,
+                                           float &fpx, float &fpy, float &fpz, float &fvx, float &fvy, float &fvz)
+{
+    float dx, dy, dz, vjx, vjy, vjz, wgt, l;
+    mixed_factors(gi, qs, r, mc, dx, dy, dz, vjx, vjy, vjz, wgt, l);
     fpx += wgt * dx;
     fpy += wgt * dy;
     fpz += wgt * dz;
-    const float l = mc.visc_q * (1.0f / INV_SCALE) * hr * qv.y;
     fvx += (vjx - vi.x) * l;
-    fvy += (vyz.x - vi.y) * l;
-    fvz += (vyz.y - vi.z) * l;
+    fvy += (vjy - vi.y) * l;
+    fvz += (vjz - vi.z) * l;
+}
+
+// The rest of the force pass for one particle: x' = x + (v dt + (a dt) dt) with x = hi + lo carried by
+// TwoSum, v' = increment / dt, and the cell of the new position.
+__device__ __forceinline__ void finish_mixed(uint32_t i, const Vec4<float> &pi, const Vec4<float> &vi, float rho,
+                                             const SceneDev &sc, const Vec4<float> *__restrict__ lo_s,
+                                             const ObstacleDev *__restrict__ obstacles, const Consts<float> &c,
+                                             float fpx, float fpy, float fpz, float fvx, float fvy, float fvz,
+                                             Vec4<float> *__restrict__ pos_out, Vec4<float> *__restrict__ lo_out,
+                                             Vec4<float> *__restrict__ vel_out, Vec4<float> *__restrict__ acc_out,
+                                             uint2 *__restrict__ cid_out, uint32_t *__restrict__ count)
+{
+    float ax, ay, az;
+    accel_of<float>(pi, vi, rho, sc, obstacles, c, fpx, fpy, fpz, fvx, fvy, fvz, ax, ay, az);
+    const Vec4<float> li = ld4(lo_s + i);
+    const float dt = c.dt;
+    const float ix = __fadd_rn(__fmul_rn(vi.x, dt), __fmul_rn(__fmul_rn(ax, dt), dt));
+    const float iy = __fadd_rn(__fmul_rn(vi.y, dt), __fmul_rn(__fmul_rn(ay, dt), dt));
+    const float iz = __fadd_rn(__fmul_rn(vi.z, dt), __fmul_rn(__fmul_rn(az, dt), dt));
+    float hx, lx, hy, ly, hz, lz;
+    two_sum(pi.x, __fadd_rn(li.x, ix), hx, lx);
+    two_sum(pi.y, __fadd_rn(li.y, iy), hy, ly);
+    two_sum(pi.z, __fadd_rn(li.z, iz), hz, lz);
+    st4(pos_out + i, Vec4<float>{hx, hy, hz, pi.w});
+    st4(lo_out + i, Vec4<float>{lx, ly, lz, 0.0f});
+    st4(vel_out + i, Vec4<float>{__fdiv_rn(ix, dt), __fdiv_rn(iy, dt), __fdiv_rn(iz, dt), vi.w});
+    if (acc_out) st4(acc_out + i, Vec4<float>{ax, ay, az, 0.0f});
+    int qx, qy, qz;
+    const uint32_t cell = hash_cell<float>(sc, hx, hy, hz, c, qx, qy, qz);
+    count_add(count, c.gsum, cell);
+    cid_out[i] = make_uint2(cell, wbits(vi.w));
 }
 
 // Two accepted neighbours per iteration: both records are loaded before either's terms are
@@ -276,26 +318,193 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_forces_mixed(
     }
     // the scene record again rather than kept live across the pair loop (fewer registers)
     const SceneDev sc2 = load_scene(scenes, wbits(pi.w));
-    float ax, ay, az;
-    accel_of<float>(pi, vi, ai.x, sc2, obstacles, c, fpx, fpy, fpz, fvx, fvy, fvz, ax, ay, az);
-    // x' = x + (v dt + (a dt) dt) with x = hi + lo carried by TwoSum; v' = increment / dt
-    const Vec4<float> li = ld4(lo_s + i);
-    const float dt = c.dt;
-    const float ix = __fadd_rn(__fmul_rn(vi.x, dt), __fmul_rn(__fmul_rn(ax, dt), dt));
-    const float iy = __fadd_rn(__fmul_rn(vi.y, dt), __fmul_rn(__fmul_rn(ay, dt), dt));
-    const float iz = __fadd_rn(__fmul_rn(vi.z, dt), __fmul_rn(__fmul_rn(az, dt), dt));
-    float hx, lx, hy, ly, hz, lz;
-    two_sum(pi.x, __fadd_rn(li.x, ix), hx, lx);
-    two_sum(pi.y, __fadd_rn(li.y, iy), hy, ly);
-    two_sum(pi.z, __fadd_rn(li.z, iz), hz, lz);
-    st4(pos_out + i, Vec4<float>{hx, hy, hz, pi.w});
-    st4(lo_out + i, Vec4<float>{lx, ly, lz, 0.0f});
-    st4(vel_out + i, Vec4<float>{__fdiv_rn(ix, dt), __fdiv_rn(iy, dt), __fdiv_rn(iz, dt), vi.w});
-    if (acc_out) st4(acc_out + i, Vec4<float>{ax, ay, az, 0.0f});
-    int qx, qy, qz;
-    const uint32_t cell = hash_cell<float>(sc2, hx, hy, hz, c, qx, qy, qz);
-    count_add(count, c.gsum, cell);
-    cid_out[i] = make_uint2(cell, wbits(vi.w));
+    finish_mixed(i, pi, vi, ai.x, sc2, lo_s, obstacles, c, fpx, fpy, fpz, fvx, fvy, fvz, pos_out, lo_out, vel_out,
+                 acc_out, cid_out, count);
+}
+
+// ---- group forms (sph_group.cuh): G lanes a particle, on cells of size h -----------------------
+// The list holds h^2 - r^2 of the accepted neighbours, in order; the first entry of every 32-candidate
+// word carries a negative sign (a word without neighbours has one entry, -0), since the words are
+// summed one by one and added with Kahan compensation.
+template <int G>
+__global__ void __launch_bounds__(kGroupThreads) k_density_group_mixed(
+    const Vec4<float> *__restrict__ pos, const uint2 *__restrict__ gpos, Vec4<float> *__restrict__ aux,
+    const uint32_t *__restrict__ start, const SceneDev *__restrict__ scenes, uint32_t n, Consts<float> c, MixConsts mc,
+    uint32_t *__restrict__ masks, const Vec4<float> *__restrict__ vel, uint4 *__restrict__ rec)
+{
+    __shared__ float list[kGroupThreads / 32][Group<G>::PER_WARP][kListLen];
+    chain_wait();
+    const Group<G> g;
+    const uint32_t i = g.particle();
+    if (i - (uint32_t) g.slot >= n) return;  // the whole warp
+    const bool live = i < n;
+    const uint32_t ic = live ? i : n - 1;
+    const Vec4<float> pi = ld4(pos + ic);
+    const uint2 gi = __ldg(gpos + ic);
+    const SceneDev sc = load_scene(scenes, wbits(pi.w));
+    int cx, cy, cz;
+    hash_cell<float>(sc, pi.x, pi.y, pi.z, c, cx, cy, cz);
+    const GroupRows<G> rows(g, sc, start, cx, cy, cz, live, n);
+    float *const mine = list[g.warp][g.slot];
+    float sum = 0, comp = 0, csum = 0;
+    bool open = false;
+    uint32_t cnt = 0;
+    auto work_off = [&]() {
+        __syncwarp();
+        if (g.gl == 0) {
+#pragma unroll 4
+            for (uint32_t k = 0; k < cnt; k++) {
+                const float v = mine[k];
+                if (__float_as_int(v) < 0) {  // a word begins
+                    if (open) kahan_add(sum, comp, csum);
+                    csum = 0;
+                    open = true;
+                }
+                csum = poly6_acc<float>(csum, fabsf(v));
+            }
+        }
+        cnt = 0;
+        __syncwarp();
+    };
+    rows.each([&](int r, uint32_t jb, uint32_t len, uint32_t most) {
+        int w = 0;
+        for (uint32_t cb = 0; cb < most; cb += 32, w++) {
+            if (__any_sync(kFullWarp, cnt > kListFlush)) work_off();
+            uint32_t m = 0;  // the word of these 32 candidates, as the other forms record it
+            const uint32_t word = cnt;
+#pragma unroll
+            for (int u = 0; u < 32 / G; u++) {
+                const uint32_t o = cb + (uint32_t) u * G + g.gl;
+                if (cb + (uint32_t) u * G >= most) break;
+                float t = 0;
+                if (o < len) {
+                    float x, y, z;
+                    code_delta(gi, __ldg(gpos + jb + o), x, y, z);
+                    t = h2_minus_r2<float>(x, y, z, QH2);
+                }
+                const unsigned hit = g.vote(t > 0);
+                if (t > 0) {
+                    const uint32_t k = cnt + (uint32_t) __popc(hit & g.below);
+                    mine[k] = k == word ? -t : t;
+                }
+                cnt += __popc(hit);
+                m |= hit << ((u * G) & 31);
+            }
+            if (m == 0 && cb < len) {
+                if (g.gl == 0) mine[cnt] = -0.0f;
+                cnt++;
+            }
+            if (g.gl == 0 && cb < len && w < Stencil<1>::WORDS)
+                masks[(size_t) (r * Stencil<1>::WORDS + w) * n + i] = m;
+        }
+    });
+    work_off();
+    if (g.gl != 0 || !live) return;
+    if (open) kahan_add(sum, comp, csum);
+    const float rho = __fmul_rn(__fmul_rn(sum, mc.poly6_q), c.mass);
+    const float p = __fmul_rn(c.k, __fsub_rn(rho, c.rho0));
+    const float q = __fdiv_rn(p, __fmul_rn(rho, rho)), inv = __fdiv_rn(1.0f, rho);
+    st4(aux + i, Vec4<float>{rho, p, q, inv});
+    const Vec4<float> vi = ld4(vel + i);
+    rec[i] = make_record(gi, vi.x, vi.y, vi.z, q, inv);
+}
+
+template <int G>
+__global__ void __launch_bounds__(kGroupThreads) k_forces_group_mixed(
+    const Vec4<float> *__restrict__ pos, const Vec4<float> *__restrict__ lo_s, const Vec4<float> *__restrict__ vel,
+    const Vec4<float> *__restrict__ aux, const uint2 *__restrict__ gpos, const uint4 *__restrict__ rec,
+    const uint32_t *__restrict__ start, const SceneDev *__restrict__ scenes, const ObstacleDev *__restrict__ obstacles,
+    uint32_t n, Consts<float> c, MixConsts mc, const uint32_t *__restrict__ masks, Vec4<float> *__restrict__ pos_out,
+    Vec4<float> *__restrict__ lo_out, Vec4<float> *__restrict__ vel_out, Vec4<float> *__restrict__ acc_out,
+    uint2 *__restrict__ cid_out, uint32_t *__restrict__ count)
+{
+    constexpr int AHEAD = G <= 8 ? 16 / G : 1;
+    constexpr int WORDS = Stencil<1>::WORDS;
+    __shared__ uint32_t list[kGroupThreads / 32][Group<G>::PER_WARP][kListLen];
+    __shared__ PairOut<float> outs[kGroupThreads / 32][Group<G>::PER_WARP][AHEAD * G];
+    __shared__ GroupSums<float, G> sums;
+    chain_wait();
+    const Group<G> g;
+    const uint32_t i = g.particle();
+    const bool live = i < n;
+    const uint32_t ic = live ? i : n - 1;
+    const Vec4<float> pi = ld4(pos + ic);
+    const Vec4<float> vi = ld4(vel + ic);
+    const float qs = ld4(aux + ic).z * Q_SCALE;
+    const uint2 gi = __ldg(gpos + ic);
+    const SceneDev sc = load_scene(scenes, wbits(pi.w));
+    int cx, cy, cz;
+    hash_cell<float>(sc, pi.x, pi.y, pi.z, c, cx, cy, cz);
+    const GroupRows<G> rows(g, sc, start, cx, cy, cz, live, n);
+    uint32_t *const mine = list[g.warp][g.slot];
+    PairOut<float> *const out = outs[g.warp][g.slot];
+    float fp = 0, fv = 0;
+    uint32_t cnt = 0;
+    auto work_off = [&]() {
+        __syncwarp();
+        const uint32_t most = __reduce_max_sync(kFullWarp, cnt);
+        for (uint32_t k0 = 0; k0 < most; k0 += AHEAD * G) {
+            uint4 rj[AHEAD];
+#pragma unroll
+            for (int a = 0; a < AHEAD; a++) {
+                const uint32_t k = k0 + (uint32_t) a * G + g.gl;
+                rj[a] = __ldg(rec + (k < cnt ? mine[k] : ic));
+            }
+#pragma unroll
+            for (int a = 0; a < AHEAD; a++) {
+                PairOut<float> o;
+                mixed_factors(gi, qs, rj[a], mc, o.v[0], o.v[2], o.v[4], o.v[1], o.v[3], o.v[5], o.v[6], o.v[7]);
+                o.v[1] -= vi.x;
+                o.v[3] -= vi.y;
+                o.v[5] -= vi.z;
+                float4 *dst = reinterpret_cast<float4 *>(out + a * G + g.gl);
+                dst[0] = make_float4(o.v[0], o.v[1], o.v[2], o.v[3]);
+                dst[1] = make_float4(o.v[4], o.v[5], o.v[6], o.v[7]);
+            }
+            __syncwarp();
+            if (g.gl < 3 && k0 < cnt) add_pairs<float>(out, min(cnt - k0, (uint32_t) (AHEAD * G)), g.gl, fp, fv);
+            __syncwarp();
+        }
+        cnt = 0;
+    };
+    rows.each([&](int r, uint32_t jb, uint32_t len, uint32_t most) {
+        int w = 0;
+        for (uint32_t cb = 0; cb < most; cb += 32, w++) {
+            if (__any_sync(kFullWarp, cnt > kListFlush)) work_off();
+            uint32_t m = 0;
+            if (w < WORDS) {
+                if (cb < len) m = __ldg(masks + (size_t) (r * WORDS + w) * n + ic);
+            } else {  // beyond the recorded words: test the candidates here
+#pragma unroll
+                for (int u = 0; u < 32 / G; u++) {
+                    const uint32_t o = cb + (uint32_t) u * G + g.gl;
+                    float t = 0;
+                    if (o < len) {
+                        float x, y, z;
+                        code_delta(gi, __ldg(gpos + jb + o), x, y, z);
+                        t = h2_minus_r2<float>(x, y, z, QH2);
+                    }
+                    m |= g.vote(t > 0) << ((u * G) & 31);
+                }
+            }
+            if (i - (jb + cb) < 32u) m &= ~(1u << (i - (jb + cb)));  // the particle itself
+#pragma unroll
+            for (int u = 0; u < 32 / G; u++) {
+                const uint32_t bit = (uint32_t) u * G + g.gl;
+                if (((m >> bit) & 1u) && sph_check(cb + bit < len, CHK_NEIGHBOUR))
+                    mine[cnt + __popc(m & ((1u << bit) - 1u))] = jb + cb + bit;
+            }
+            cnt += __popc(m);
+        }
+    });
+    work_off();
+    sums.put(g, fp, fv);
+    const uint32_t k = threadIdx.x, e = blockIdx.x * Group<G>::PER_BLOCK + k;
+    if (k >= (uint32_t) Group<G>::PER_BLOCK || e >= n) return;
+    const Vec4<float> pe = ld4(pos + e);
+    finish_mixed(e, pe, ld4(vel + e), ld4(aux + e).x, load_scene(scenes, wbits(pe.w)), lo_s, obstacles, c, sums.f[k][0], sums.f[k][1],
+                 sums.f[k][2], sums.f[k][3], sums.f[k][4], sums.f[k][5], pos_out, lo_out, vel_out, acc_out, cid_out,
+                 count);
 }
 
 // ---- egress: id-ordered hi + lo positions (float or double), velocities, rho, p ---------
@@ -349,10 +558,35 @@ cudaError_t mixed_permute(const DevBufs &b, uint32_t n, Consts<float> c, MixCons
                           b.gpos, b.big);
 }
 
+// Where the group forms are used: as for the plain form (group_density). Density and forces together, in
+// us, with 16 lanes, 8 lanes and one thread a particle: 2,000 at rest 25 / 27 / 41, 8,000 fallen 35 / 39 /
+// 70, 20,000 fallen 59 / 49 / 80, 40,000 fallen 94 / 82 / 84, 61,000 at rest 94 / 70 / 47.
+template <int G>
+static cudaError_t mixed_density_g(const DevBufs &b, uint32_t n, Consts<float> c, MixConsts mc, cudaStream_t st)
+{
+    return launch_chained(k_density_group_mixed<G>, nblk(n, Group<G>::PER_BLOCK), kGroupThreads, st,
+                          (const Vec4<float> *) b.pos_s, b.gpos, (Vec4<float> *) b.aux, b.start, b.scenes, n, c, mc,
+                          b.masks, (const Vec4<float> *) b.vel_s, (uint4 *) b.frec);
+}
+
+template <int G>
+static cudaError_t mixed_forces_g(const DevBufs &b, uint32_t n, Consts<float> c, MixConsts mc, bool record_acc,
+                                  cudaStream_t st)
+{
+    return launch_chained(
+        k_forces_group_mixed<G>, nblk(n, Group<G>::PER_BLOCK), kGroupThreads, st, (const Vec4<float> *) b.pos_s,
+        (const Vec4<float> *) b.lo_s, (const Vec4<float> *) b.vel_s, (const Vec4<float> *) b.aux, b.gpos,
+        (const uint4 *) b.frec, b.start, b.scenes, b.obstacles, n, c, mc, b.masks, (Vec4<float> *) b.pos_u,
+        (Vec4<float> *) b.lo_u, (Vec4<float> *) b.vel_u,
+        record_acc ? (Vec4<float> *) b.acc : (Vec4<float> *) nullptr, b.cid_u, b.count);
+}
+
 cudaError_t mixed_density(const DevBufs &b, uint32_t n, Consts<float> c, MixConsts mc, int cell_mult,
                           cudaStream_t st)
 {
     if (!n) return cudaSuccess;
+    if (cell_mult == 1 && n <= kGroupMax)
+        return n <= kGroupWide ? mixed_density_g<16>(b, n, c, mc, st) : mixed_density_g<8>(b, n, c, mc, st);
     // blocks of 128: the SMs finish the dense and sparse regions more evenly than with 256
     return launch_chained(cell_mult == 2 ? k_density_mixed<2> : k_density_mixed<1>, nblk(n, 128), 128, st,
                           (const Vec4<float> *) b.pos_s, b.gpos, (Vec4<float> *) b.aux, b.start, b.scenes, n, c, mc,
@@ -389,6 +623,9 @@ cudaError_t mixed_forces(const DevBufs &b, uint32_t n, Consts<float> c, MixConst
                          int cell_mult, cudaStream_t st)
 {
     if (!n) return cudaSuccess;
+    if (cell_mult == 1 && variant == 0 && n <= kGroupMax)
+        return n <= kGroupWide ? mixed_forces_g<16>(b, n, c, mc, record_acc, st)
+                               : mixed_forces_g<8>(b, n, c, mc, record_acc, st);
     return cell_mult == 2 ? mixed_forces_rad<2>(b, n, c, mc, record_acc, variant, st)
                           : mixed_forces_rad<1>(b, n, c, mc, record_acc, variant, st);
 }

@@ -66,6 +66,26 @@ def test_f64_group_form_equals_one_thread_forms(sphlib, n, kind):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,kind", [(1, "lattice"), (35, "clump"), (1501, "clump"), (10240, "clump"),
+                                    (10241, "lattice"), (32768, "lattice"), (32769, "clump")])
+def test_mixed_group_form_equals_one_thread_form(sphlib, n, kind):
+    """The mixed form's density sums are compensated word by word: the group form must keep each word's
+    sum and their order. A context of two scenes that together exceed the group form's range runs the
+    one-thread kernels on the same particles."""
+    box, pos, vel = scene(n, kind, 7)
+    got = run(sphlib, box, pos, vel, None, sphlib.SPH_MIXED)
+    filler, fpos, fvel = scene(33000, "lattice", 8)
+    ctx = sphlib.SphContext([box, filler], [n, 33000], gravity=G981, flags=sphlib.SPH_FLAG_RECORD_ACC,
+                            precision=sphlib.SPH_MIXED)
+    ctx.upload(np.concatenate([pos, fpos]), np.concatenate([vel, fvel]), [n, 33000])
+    ctx.step(3)
+    ref = ctx.download(acc=True)
+    ctx.close()
+    for k in got:
+        assert np.array_equal(got[k], ref[k][:n]), (n, kind, k)
+
+
+@pytest.mark.gpu
 def test_f64_far_coordinates(sphlib):
     """Coordinates whose float rounding is larger than h, beyond the float range of squares, and
     infinite: the float test decides nothing there and the exact one gives the mask form's bits."""
