@@ -67,6 +67,7 @@ struct sph_ctx {
     uint32_t graph_n = 0;
     std::vector<uint32_t> scene_off_host;
     Tune tune;
+    bool quads = false;        // st_xyz holds the sorted positions' quads (written by the last grid pass)
     int dense_mode = 3;        // force variant that the last density pass prepared for
     bool tune_pinned = false;  // variants set explicitly: the cache does not override them
     bool cell_pinned = false;  // cell multiple set explicitly: the autotuner keeps it
@@ -271,8 +272,8 @@ size_t pool_layout(sph_ctx *c, std::vector<PoolItem> &items)
         {(void **) &b.bsum, 4 * nb}, {(void **) &b.big, 4 * big_words(N)},
         {(void **) &b.scenes, sizeof(SceneDev) * c->sc.size()},
         {(void **) &b.obstacles, sizeof(ObstacleDev) * (nobs ? nobs : 1)},
-        {(void **) &b.scene_off, 4 * (c->sc.size() + 1)}, {(void **) &b.err, 16},
-        {(void **) &b.st_xyz, 12 * N}, {(void **) &b.st_vel, 12 * N},
+        {(void **) &b.scene_off, 4 * (c->sc.size() + 1)},
+        {(void **) &b.st_xyz, 12 * N + 48}, {(void **) &b.st_vel, 12 * N},
         {(void **) &b.st_rho, rs == 4 ? 4 * N : 0}, {(void **) &b.st_p, rs == 4 ? 4 * N : 0},
         {(void **) &b.st_acc, rs == 4 && rec ? 12 * N : 0},
         {(void **) &b.st_xyz64, (rs == 8 || mixed) ? 24 * N : 0}, {(void **) &b.st_vel64, (rs == 8 || mixed) ? 24 * N : 0},
@@ -325,7 +326,6 @@ int allocate(sph_ctx *c)
     }
     if (int rc = clear_counts(c, C)) return rc;
     CK(c, cudaMemsetAsync(b.aux, 0, r4 * N, c->stream));
-    CK(c, cudaMemsetAsync(b.err, 0, 16, c->stream));
     return SPH_OK;
 }
 
@@ -469,7 +469,11 @@ int run_grid(sph_ctx *c)
         CK(c, launch_slot(c->b, c->n, (uint32_t) c->ctot, c->stream));
         CK(c, mixed_permute(c->b, c->n, make_consts<float>(c, c->tune.cell_mult), make_mix(c->prm), c->stream));
     } else {
-        CK(c, Launch<R>::permute(c->b, c->n, (uint32_t) c->ctot, c->stream));
+        // quads for the density pass of the record variants on cells of size h (smaller scenes of the
+        // default variant take the group form)
+        const int f = c->tune.forces_mode;
+        c->quads = !is_f64(c) && c->tune.cell_mult == 1 && ((f >= 7 && f <= 11) || (f == 3 && c->n > kGroupMax));
+        CK(c, Launch<R>::permute(c->b, c->n, (uint32_t) c->ctot, c->quads, c->stream));
     }
     return SPH_OK;
 }
@@ -479,7 +483,7 @@ int run_density(sph_ctx *c)
     if (is_mixed(c))
         CK(c, mixed_density(c->b, c->n, make_consts<float>(c, c->tune.cell_mult), make_mix(c->prm),
                             c->tune.cell_mult, c->stream));
-    else CK(c, Launch<R>::density(c->b, c->n, make_consts<R>(c, c->tune.cell_mult), c->tune, c->stream));
+    else CK(c, Launch<R>::density(c->b, c->n, make_consts<R>(c, c->tune.cell_mult), c->tune, c->quads, c->stream));
     c->dense_mode = c->tune.forces_mode;
     return SPH_OK;
 }
@@ -1206,6 +1210,10 @@ int sph_autotune(sph_ctx *c, int32_t reps)
             int rc = set_cell_mult(c, m);
             if (rc) return rc;
         }
+        if (!is_mixed(c)) {  // a variant whose grid pass also writes what the record variants read
+            c->tune.density_p = 0;
+            c->tune.forces_mode = 7;
+        }
         CK(c, cudaEventRecord(c->ev[0], c->stream));
         int rc = pass_grid(c);
         if (rc) return rc;
@@ -1337,6 +1345,7 @@ static int download_impl(sph_ctx *c, void *xyz, void *vel, void *rho, void *p, v
     void *sr = f64 ? (void *) b.st_rho64 : (void *) b.st_rho;
     void *sp = f64 ? (void *) b.st_p64 : (void *) b.st_p;
     void *sa = f64 ? (void *) b.st_acc64 : (void *) b.st_acc;
+    c->quads = false;  // the staging arrays are written now
     CK(c, cudaMemsetAsync(sr, 0, rs * n, c->stream));
     CK(c, cudaMemsetAsync(sp, 0, rs * n, c->stream));
     if (sa) CK(c, cudaMemsetAsync(sa, 0, 3 * rs * n, c->stream));
@@ -1518,6 +1527,7 @@ namespace {
 int get_grid_ref(sph_ctx *c, uint32_t *cell_of_particle, uint32_t *cell_counts, uint32_t *sorted_ids)
 {
     const uint32_t n = c->n;
+    c->quads = false;  // the staging arrays are written now
     // id-ordered float positions of the sorted state (the mixed form's hi part: its hash input)
     if (is_mixed(c)) CK(c, mixed_egress(c->b, n, 0, 0, 1, 1, false, c->stream));
     else CK(c, Launch<float>::egress(c->b, n, 0, 0, 1, 1, c->stream));

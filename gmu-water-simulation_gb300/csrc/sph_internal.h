@@ -64,8 +64,8 @@ struct DevBufs {
     SceneDev *scenes;
     ObstacleDev *obstacles;
     uint32_t *scene_off;   // first output index of every scene (id-order downloads)
-    int32_t *err;          // device error flag
-    // staging for host transfers (ingest / egress)
+    // staging for host transfers (ingest / egress); between a grid pass and its density pass st_xyz also
+    // holds rounded positions (FP64) or quads of positions (plain)
     float *st_xyz, *st_vel, *st_rho, *st_p, *st_acc;
     double *st_xyz64, *st_vel64, *st_rho64, *st_p64, *st_acc64;
     double *stats;         // per-scene FP64 reductions, 8 doubles each
@@ -142,6 +142,7 @@ struct MixConsts {
 //   cell_mult : the step grid's cells are h / cell_mult wide (1 or 2); the neighbour passes walk
 //               (2 cell_mult + 1)^2 rows of 2 cell_mult + 1 cells (only the mask-driven record
 //               variants, 7 to 11 and the mixed form's, run on cells of h/2)
+constexpr uint32_t kRecordsCapped = 524288;
 struct Tune {
     static constexpr int ALL_PAIRS = 16;  // both passes over every particle of the scene
     int density_p = 2;
@@ -183,11 +184,14 @@ struct Launch {
     static cudaError_t ingest(const DevBufs &b, const float *xyz, const float *vel, uint32_t first, uint32_t n,
                               int32_t scene, uint32_t id0, uint32_t nscenes, Consts<R> c, cudaStream_t st);
     static cudaError_t scan(const DevBufs &b, uint32_t ncells, cudaStream_t st);
-    static cudaError_t permute(const DevBufs &b, uint32_t n, uint32_t ncells, cudaStream_t st);
+    // quads: also the positions as quads of four, in st_xyz (plain form)
+    static cudaError_t permute(const DevBufs &b, uint32_t n, uint32_t ncells, bool quads, cudaStream_t st);
     // positions of the first n *_u particles hashed again into the step grid (after the cell
     // multiple changed): counts and the cells of cid_u
     static cudaError_t rehash(const DevBufs &b, uint32_t n, Consts<R> c, cudaStream_t st);
-    static cudaError_t density(const DevBufs &b, uint32_t n, Consts<R> c, const Tune &t, cudaStream_t st);
+    // quads: st_xyz holds this state's quads
+    static cudaError_t density(const DevBufs &b, uint32_t n, Consts<R> c, const Tune &t, bool quads,
+                               cudaStream_t st);
     static cudaError_t forces(const DevBufs &b, uint32_t n, Consts<R> c, bool record_acc, const Tune &t,
                               cudaStream_t st);
     // state of the first n_state particles, density/pressure of the first n_aux, and

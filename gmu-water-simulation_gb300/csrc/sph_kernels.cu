@@ -290,6 +290,11 @@ __global__ void __launch_bounds__(256) k_rank_permute(const uint2 *__restrict__ 
         posf[3 * (size_t) dst] = (float) p.x;
         posf[3 * (size_t) dst + 1] = (float) p.y;
         posf[3 * (size_t) dst + 2] = (float) p.z;
+    } else if (posf) {  // quads of positions for the density pass (k_density_quad)
+        float *q = posf + 12 * (size_t) (dst >> 2) + (dst & 3u);
+        q[0] = p.x;
+        q[4] = p.y;
+        q[8] = p.z;
     }
 }
 
@@ -496,15 +501,137 @@ __global__ void __launch_bounds__(256) k_density_mask(const Vec4<R> *__restrict_
     }
 }
 
+// Density with masks and records from quads of positions: the grid pass also writes the sorted positions
+// as 48-byte groups of four, x0..x3 y0..y3 z0..z3 (cells of size h only: the rows of cells of h/2 are too
+// short for it). The kernel with one 16-byte load per candidate (k_density_mask) is held by the load path
+// as much as by issue: a warp's 16-byte load takes 4 cycles of it even where the lanes share an address
+// (70% of its peak at 85% of the issue slots). Three loads now bring four candidates, and pairs of
+// candidates share packed FP32x2 arithmetic, which saves instructions but not dispatch slots (a packed
+// instruction takes two). Bound by those: 99M instructions, 26M of them packed, instead of 124M for
+// 1,000,000 particles at rest, 121 us instead of 127 (fallen 217 / 237; 300,000 at rest 45 / 72, 61,000
+// fallen 29 / 37, where the longer independent runs per row also hide more latency).
+//
+// The same bits as k_density_mask: the differences and h^2 - r^2 enter with the opposite sign, which
+// rounds alike, and the accepted terms are added one by one in candidate order. A row is walked from the
+// quad that holds its first candidate to the quad that holds its last; those two quads also hold other
+// rows' particles and check each candidate (CHECK), the quads between them need not.
+template <bool CHECK>
+__device__ __forceinline__ void density_quad(const float4 *__restrict__ p, uint32_t o, uint32_t len, float2 nx, float2 ny,
+                                             float2 nz, float2 nh2, float &acc, uint32_t &word)
+{
+    const float4 X = __ldg(p), Y = __ldg(p + 1), Z = __ldg(p + 2);
+    const float2 dx = __fadd2_rn(make_float2(X.x, X.y), nx), ex = __fadd2_rn(make_float2(X.z, X.w), nx);
+    const float2 dy = __fadd2_rn(make_float2(Y.x, Y.y), ny), ey = __fadd2_rn(make_float2(Y.z, Y.w), ny);
+    const float2 dz = __fadd2_rn(make_float2(Z.x, Z.y), nz), ez = __fadd2_rn(make_float2(Z.z, Z.w), nz);
+    float2 s = __ffma2_rn(dx, dx, nh2), t = __ffma2_rn(ex, ex, nh2);  // r^2 - h^2
+    s = __ffma2_rn(dy, dy, s);
+    t = __ffma2_rn(ey, ey, t);
+    s = __ffma2_rn(dz, dz, s);
+    t = __ffma2_rn(ez, ez, t);
+    if (CHECK) {  // o: the quad's first candidate, counted from the row's first (unsigned: below it is far beyond len)
+        s.x = o < len ? s.x : 0.0f;
+        s.y = o + 1 < len ? s.y : 0.0f;
+        t.x = o + 2 < len ? t.x : 0.0f;
+        t.y = o + 3 < len ? t.y : 0.0f;
+    }
+    s.x = fminf(s.x, 0.0f);  // also a NaN's
+    s.y = fminf(s.y, 0.0f);
+    t.x = fminf(t.x, 0.0f);
+    t.y = fminf(t.y, 0.0f);
+    const float2 u = __fmul2_rn(s, s), v = __fmul2_rn(t, t);
+    acc = __fmaf_rn(u.x, -s.x, acc);
+    acc = __fmaf_rn(u.y, -s.y, acc);
+    acc = __fmaf_rn(v.x, -t.x, acc);
+    acc = __fmaf_rn(v.y, -t.y, acc);
+    word = __funnelshift_l(__float_as_uint(s.x), word, 1);  // accepted: the sign bit, entering at the bottom
+    word = __funnelshift_l(__float_as_uint(s.y), word, 1);
+    word = __funnelshift_l(__float_as_uint(t.x), word, 1);
+    word = __funnelshift_l(__float_as_uint(t.y), word, 1);
+}
+
+// One row of len candidates from jb on; its words of accepted candidates, counted from jb, to out.
+__device__ __forceinline__ void density_row(const float4 *__restrict__ quads, uint32_t jb, uint32_t len, float2 nx,
+                                            float2 ny, float2 nz, float2 nh2, float &acc, uint32_t *__restrict__ out,
+                                            uint32_t stride, int words, uint64_t keep)
+{
+    const uint32_t lead = jb & 3u, last = (lead + len - 1u) >> 2;  // last quad
+    const float4 *p = quads + 3 * (size_t) (jb >> 2);
+    uint32_t before = 0, word = 0;  // the previous and the current 32 bits, from the first quad's first candidate on
+    int w = -1;                     // the row's word that `before` begins
+    auto next_word = [&](uint32_t bits) {
+        word = __brev(word) >> (32u - bits);
+        if (w >= 0 && w < words) st_keep(out + (size_t) w * stride, __funnelshift_r(before, word, lead), keep);
+        before = word;
+        word = 0;
+        w++;
+    };
+    density_quad<true>(p, 0u - lead, len, nx, ny, nz, nh2, acc, word);
+    uint32_t q = 1;
+    while (q < last) {
+        const uint32_t e = min(last, (q | 7u) + 1u);
+#pragma unroll 2
+        for (; q < e; q++) density_quad<false>(p + 3 * q, 0, 0, nx, ny, nz, nh2, acc, word);
+        if ((q & 7u) == 0) next_word(32);
+    }
+    if (last > 0) density_quad<true>(p + 3 * (size_t) last, 4 * last - lead, len, nx, ny, nz, nh2, acc, word);
+    next_word(4 * (last & 7u) + 4);
+    if (w < words && 32u * (uint32_t) w < len) st_keep(out + (size_t) w * stride, before >> lead, keep);
+}
+
+__global__ void __launch_bounds__(256) k_density_quad(const Vec4<float> *__restrict__ pos,
+                                                      const float4 *__restrict__ quads, Vec4<float> *__restrict__ aux,
+                                                      const uint32_t *__restrict__ start,
+                                                      const SceneDev *__restrict__ scenes, uint32_t n, Consts<float> c,
+                                                      uint32_t *__restrict__ masks, const Vec4<float> *__restrict__ vel,
+                                                      Vec4<float> *__restrict__ frec)
+{
+    using St = Stencil<1>;
+    constexpr int RAD = 1;
+    chain_wait();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const Vec4<float> pi = ld4(pos + i);
+    const SceneDev sc = load_scene(scenes, wbits(pi.w));
+    int cx, cy, cz;
+    hash_cell<float>(sc, pi.x, pi.y, pi.z, c, cx, cy, cz);
+    const float2 nx = make_float2(-pi.x, -pi.x), ny = make_float2(-pi.y, -pi.y), nz = make_float2(-pi.z, -pi.z);
+    const float2 nh2 = make_float2(-c.h2, -c.h2);
+    float acc = 0;
+    const uint64_t keep = l2_keep_policy();  // masks and records: read by the force pass next
+    const int X = sc.res[0], Y = sc.res[1], Z = sc.res[2];
+    const int xl = cx - RAD > 0 ? cx - RAD : 0, xh = cx + RAD < X ? cx + RAD : X - 1;
+#pragma unroll 1
+    for (int dz = -RAD; dz <= RAD; dz++) {
+#pragma unroll 1
+        for (int dy = -RAD; dy <= RAD; dy++) {
+            const int r = (dz + RAD) * (2 * RAD + 1) + (dy + RAD);
+            const int z = cz + dz, y = cy + dy;
+            if (z < 0 || z >= Z || y < 0 || y >= Y) continue;
+            const uint32_t row = sc.cell_base + (uint32_t) y * (uint32_t) X + (uint32_t) z * (uint32_t) X * (uint32_t) Y;
+            const uint32_t jb = __ldg(start + row + xl), je = __ldg(start + row + xh + 1);
+            if (!sph_check(jb <= je && je <= n, CHK_ROW) || jb == je) continue;
+            density_row(quads, jb, je - jb, nx, ny, nz, nh2, acc, masks + (size_t) (r * St::WORDS) * n + i, n, St::WORDS,
+                        keep);
+        }
+    }
+    const float rho = rmul(rmul(acc, c.c_poly6), c.mass);
+    const float p = rmul(c.k, rsub(rho, c.rho0));
+    const Vec4<float> ar = aux_record<float>(rho, p, c);
+    st4(aux + i, ar);
+    const Vec4<float> vi = ld4(vel + i);
+    st4_keep(frec + 2 * (size_t) i, Vec4<float>{pi.x, pi.y, pi.z, ar.z}, keep);
+    st4_keep(frec + 2 * (size_t) i + 1, Vec4<float>{vi.x, vi.y, vi.z, ar.w}, keep);
+}
+
 // Forces driven by the density pass's masks: only accepted neighbours are visited, in the
 // same candidate order as the scanning forms (so the sums are bit-identical).
-template <class R, int MINB, bool REC>
-__global__ void __launch_bounds__(256, MINB) k_forces_mask(
+template <class R>
+__global__ void __launch_bounds__(256, 4) k_forces_mask(
     const Vec4<R> *__restrict__ pos, const Vec4<R> *__restrict__ vel, const Vec4<R> *__restrict__ aux,
     const uint32_t *__restrict__ start, const SceneDev *__restrict__ scenes, const ObstacleDev *__restrict__ obstacles,
-    uint32_t n, Consts<R> c, const uint32_t *__restrict__ masks, const Vec4<R> *__restrict__ frec,
-    Vec4<R> *__restrict__ pos_out, Vec4<R> *__restrict__ vel_out, Vec4<R> *__restrict__ acc_out,
-    uint2 *__restrict__ cid_out, uint32_t *__restrict__ count)
+    uint32_t n, Consts<R> c, const uint32_t *__restrict__ masks, Vec4<R> *__restrict__ pos_out,
+    Vec4<R> *__restrict__ vel_out, Vec4<R> *__restrict__ acc_out, uint2 *__restrict__ cid_out,
+    uint32_t *__restrict__ count)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -545,12 +672,7 @@ __global__ void __launch_bounds__(256, MINB) k_forces_mask(
                     const uint32_t j = cb + (uint32_t) (__ffs(m) - 1);
                     m &= m - 1;
                     if (j == i || !sph_check(j < je, CHK_NEIGHBOUR)) continue;
-                    if (REC) {
-                        const Vec4<R> pj = ld4(frec + 2 * (size_t) j), vj = ld4(frec + 2 * (size_t) j + 1);
-                        pair_terms<R>(pi, vi, qi, pj, vj, pj.w, vj.w, c, fpx, fpy, fpz, fvx, fvy, fvz);
-                    } else {
-                        pair_force<R>(pi, vi, qi, j, pos, vel, aux, c, fpx, fpy, fpz, fvx, fvy, fvz);
-                    }
+                    pair_force<R>(pi, vi, qi, j, pos, vel, aux, c, fpx, fpy, fpz, fvx, fvy, fvz);
                 }
             }
         }
@@ -957,14 +1079,14 @@ cudaError_t Launch<R>::scan(const DevBufs &b, uint32_t ncells, cudaStream_t st)
 }
 
 template <class R>
-cudaError_t Launch<R>::permute(const DevBufs &b, uint32_t n, uint32_t ncells, cudaStream_t st)
+cudaError_t Launch<R>::permute(const DevBufs &b, uint32_t n, uint32_t ncells, bool quads, cudaStream_t st)
 {
     if (!n) return cudaSuccess;
     cudaError_t e = launch_slot(b, n, ncells, st);
     if (e != cudaSuccess) return e;
     return launch_chained(k_rank_permute<R>, nblk(n, 256), 256, st, b.cid_u, n, b.start, b.tmp,
                           (const Vec4<R> *) b.pos_u, (const Vec4<R> *) b.vel_u, (Vec4<R> *) b.pos_s,
-                          (Vec4<R> *) b.vel_s, b.big, b.st_xyz);
+                          (Vec4<R> *) b.vel_s, b.big, quads || sizeof(R) == 8 ? b.st_xyz : (float *) nullptr);
 }
 
 template <class R>
@@ -977,7 +1099,7 @@ cudaError_t Launch<R>::rehash(const DevBufs &b, uint32_t n, Consts<R> c, cudaStr
 }
 
 template <class R>
-cudaError_t Launch<R>::density(const DevBufs &b, uint32_t n, Consts<R> c, const Tune &t, cudaStream_t st)
+cudaError_t Launch<R>::density(const DevBufs &b, uint32_t n, Consts<R> c, const Tune &t, bool quads, cudaStream_t st)
 {
     if (!n) return cudaSuccess;
     const Vec4<R> *pos = (const Vec4<R> *) b.pos_s;
@@ -988,7 +1110,11 @@ cudaError_t Launch<R>::density(const DevBufs &b, uint32_t n, Consts<R> c, const 
     }
     if (t.forces_mode == 3 && t.cell_mult == 1 && (sizeof(R) == 8 || n <= kGroupMax))
         return group_density(b, n, c, st);
-    if (t.forces_mode >= 7) {  // masks and force records
+    if (t.forces_mode >= 7 || t.forces_mode == 3) {  // masks and force records
+        if constexpr (sizeof(R) == 4)
+            if (quads && t.cell_mult == 1)
+                return launch_chained(k_density_quad, nblk(n, 256), 256, st, pos, (const float4 *) b.st_xyz, aux,
+                                      b.start, b.scenes, n, c, b.masks, (const Vec4<R> *) b.vel_s, (Vec4<R> *) b.frec);
         if (t.cell_mult == 2) {
             if constexpr (sizeof(R) == 4)
                 return launch_chained(k_density_mask<R, true, 2>, nblk(n, 256), 256, st, pos, aux, b.start, b.scenes,
@@ -1002,7 +1128,7 @@ cudaError_t Launch<R>::density(const DevBufs &b, uint32_t n, Consts<R> c, const 
         return cudaGetLastError();
     }
     if (t.cell_mult != 1) return cudaErrorInvalidValue;  // cells of h/2: the record variants only
-    if (t.forces_mode >= 3) {  // the mask-driven force passes need the masks
+    if (t.forces_mode >= 4) {  // the mask-driven force passes need the masks
         k_density_mask<R, false><<<nblk(n, 256), 256, 0, st>>>(pos, aux, b.start, b.scenes, n, c, b.masks, nullptr,
                                                                nullptr);
         return cudaGetLastError();
@@ -1048,18 +1174,18 @@ cudaError_t Launch<R>::forces(const DevBufs &b, uint32_t n, Consts<R> c, bool re
         }
     }
     if (t.forces_mode == 3 && (sizeof(R) == 8 || n <= kGroupMax)) return group_forces(b, n, c, record_acc, st);
-    switch (t.forces_mode) {
+    // the default variant beyond the group form: the record kernel with no register cap while the GPU has
+    // fewer warps than it can hold, the 40-register one in blocks of 128 when it has many times more
+    // (300,000 at rest 51 / 57 us, fallen 111 / 113; 700,000 fallen 234 / 219; 1,000,000 at rest 150 / 137)
+    const int mode = t.forces_mode != 3 ? t.forces_mode : n < kRecordsCapped ? 7 : 10;
+    switch (mode) {
     case Tune::ALL_PAIRS:
         k_forces_all<R><<<nblk(n, 256), 256, 0, st>>>(pos, vel, aux, b.start, b.scenes, b.obstacles, n, c, po, vo, ao,
                                                       b.cid_u, b.count);
         break;
-    case 3:
-        k_forces_mask<R, 0, false><<<nblk(n, 256), 256, 0, st>>>(pos, vel, aux, b.start, b.scenes, b.obstacles, n,
-                                                                 c, b.masks, nullptr, po, vo, ao, b.cid_u, b.count);
-        break;
     case 4:
-        k_forces_mask<R, 4, false><<<nblk(n, 256), 256, 0, st>>>(pos, vel, aux, b.start, b.scenes, b.obstacles, n,
-                                                                 c, b.masks, nullptr, po, vo, ao, b.cid_u, b.count);
+        k_forces_mask<R><<<nblk(n, 256), 256, 0, st>>>(pos, vel, aux, b.start, b.scenes, b.obstacles, n, c, b.masks, po,
+                                                       vo, ao, b.cid_u, b.count);
         break;
     case 5:
         k_forces_mask2<R, 4, false><<<nblk(n, 256), 256, 0, st>>>(pos, vel, aux, b.start, b.scenes, b.obstacles, n,

@@ -194,7 +194,7 @@ int sph_pass_times(sph_ctx *ctx, double ms[5]);
  *            3..11 = the density pass records each particle's accepted neighbours as bit masks
  *            per row and the force pass visits only those (density_variant is then unused):
  *            3 (the default) with several lanes per particle in small scenes (plain form up to
- *            32,768 particles; FP64 form), else as 4; 4 one neighbour per iteration; 5 and 6 two per
+ *            32,768 particles; FP64 form), else as 7 or 10; 4 one neighbour per iteration; 5 and 6 two per
  *            iteration (5 capped at 64); 7 is 6 reading each neighbour from one packed 32-byte
  *            force record written by the density pass; 8 and 9 are 7 capped at 48 and 40
  *            registers (5 and 6 blocks of 256 per SM); 10 and 11 are 9 and 8 launched in
