@@ -85,7 +85,7 @@ struct sph_ctx {
     int trial_m[kOnlineMax] = {}, trial_v[kOnlineMax] = {};  // its cell multiple and force variant
     int last_best_v[3] = {0, 10, 10};  // per cell multiple, the force variant its last trials kept
     cudaEvent_t on_ev[2] = {nullptr, nullptr};
-    int graph_forces = -1;     // force variant captured in the graph
+    int graph_forces = -1, graph_density = -1;  // variants captured in the graph
     std::vector<unsigned char *> canaries;  // checked builds: the guard region after each array
 };
 
@@ -572,6 +572,7 @@ int build_graph(sph_ctx *c, int steps)
     c->graph_steps = steps;
     c->graph_n = c->n;
     c->graph_forces = c->tune.forces_mode;
+    c->graph_density = c->tune.density_p;
     return SPH_OK;
 }
 
@@ -905,7 +906,8 @@ int sph_upload(sph_ctx *c, const float *xyz, const float *vel, const uint32_t *c
         }
         if (total && !xyz) return fail(c, SPH_ERR_ARG, "xyz is NULL");
         CK(c, cudaSetDevice(c->device));
-        drop_graph(c);
+        // the step graph stays: it refers to the context's own arrays, and sph_step builds it again where the
+        // particle count or the variant it was built for differs (a new cell multiple drops it)
         for (size_t s = 0; s < c->sc.size(); s++) c->sc[s].count = counts[s];
         c->n = (uint32_t) total;
         // the cached choice of this particle-count bucket, its cell multiple before the hash
@@ -1122,7 +1124,8 @@ int sph_step(sph_ctx *c, int32_t nsteps)
                                              c->online_period - c->steps_run % (uint64_t) c->online_period);
         int k = 0;
         if (chunk >= unroll) {
-            if (!c->graph || c->graph_steps != unroll || c->graph_n != c->n || c->graph_forces != c->tune.forces_mode) {
+            if (!c->graph || c->graph_steps != unroll || c->graph_n != c->n ||
+                c->graph_forces != c->tune.forces_mode || c->graph_density != c->tune.density_p) {
                 int rc = build_graph(c, unroll);
                 if (rc) return rc;
                 c->state = HASHED;
