@@ -56,7 +56,7 @@ DIMS = (100, 100, 100)
 GRAVITY = (0.0, -9.81, 0.0)
 SEED = 1
 H32 = np.float32(0.0457)
-KERNELS_PER_STEP = 6  # scan, slot, crowded-cell sort, rank+permute, density, forces
+KERNELS_PER_STEP = 5  # scan, slot, rank+permute, density, forces
 RUN_STEPS = 500        # the configuration's run
 BATCH_RUN_STEPS = 1000  # the 256-scene batch's run
 SM_COUNT = 152
@@ -622,7 +622,7 @@ def run_config(args):
     ms = []
     work = advance(args.steps, ms)
     # five more steps from the final state (the run's largest particle count), each pass between
-    # its own events; the grid pass is the scan, slot, crowded-cell sort, rank and permute
+    # its own events; the grid pass is the scan, slot, rank and permute
     fin = []
     for _ in range(5):
         e = [torch.cuda.Event(enable_timing=True) for _ in range(4)]

@@ -125,13 +125,12 @@ MixConsts make_mix(const sph_params &p)
 }
 size_t r4_bytes(const sph_ctx *c) { return is_f64(c) ? 32 : 16; }
 
-// The hash outputs of a grid of ncells cells cleared: the per-cell counts, their per-group sums
-// and the crowded-cell list (the step's own passes leave all three empty between steps).
+// The hash outputs of a grid of ncells cells cleared: the per-cell counts and their per-group sums
+// (the step's own passes leave both empty between steps).
 int clear_counts(sph_ctx *c, uint64_t ncells)
 {
     CK(c, cudaMemsetAsync(c->b.count, 0, 4 * ncells, c->stream));
     CK(c, cudaMemsetAsync(c->b.bsum, 0, 4 * (ncells / kScanTile + 1), c->stream));
-    CK(c, cudaMemsetAsync(c->b.big, 0, 4, c->stream));
     return SPH_OK;
 }
 
@@ -269,7 +268,7 @@ size_t pool_layout(sph_ctx *c, std::vector<PoolItem> &items)
         {&b.acc, rec ? r4 * N : 0},
         {(void **) &b.cid_u, 8 * N}, {(void **) &b.tmp, 4 * N},
         {(void **) &b.count, 4 * C}, {(void **) &b.start, 4 * (C + 1)},
-        {(void **) &b.bsum, 4 * nb}, {(void **) &b.big, 4 * big_words(N)},
+        {(void **) &b.bsum, 4 * nb},
         {(void **) &b.scenes, sizeof(SceneDev) * c->sc.size()},
         {(void **) &b.obstacles, sizeof(ObstacleDev) * (nobs ? nobs : 1)},
         {(void **) &b.scene_off, 4 * (c->sc.size() + 1)},
@@ -464,17 +463,16 @@ int create_common(const sph_params *p, uint32_t n_scenes, const sph_scene_desc *
 template <class R>
 int run_grid(sph_ctx *c)
 {
-    CK(c, Launch<R>::scan(c->b, (uint32_t) c->ctot, c->stream));
     if (is_mixed(c)) {
-        CK(c, launch_slot(c->b, c->n, (uint32_t) c->ctot, c->stream));
-        CK(c, mixed_permute(c->b, c->n, make_consts<float>(c, c->tune.cell_mult), make_mix(c->prm), c->stream));
-    } else {
-        // quads for the density pass of the record variants on cells of size h (smaller scenes of the
-        // default variant take the group form)
-        const int f = c->tune.forces_mode;
-        c->quads = !is_f64(c) && c->tune.cell_mult == 1 && ((f >= 7 && f <= 11) || (f == 3 && c->n > kGroupMax));
-        CK(c, Launch<R>::permute(c->b, c->n, (uint32_t) c->ctot, c->quads, c->stream));
+        CK(c, mixed_grid(c->b, c->n, (uint32_t) c->ctot, make_consts<float>(c, c->tune.cell_mult), make_mix(c->prm),
+                         c->stream));
+        return SPH_OK;
     }
+    // quads for the density pass of the record variants on cells of size h (smaller scenes of the
+    // default variant take the group form)
+    const int f = c->tune.forces_mode;
+    c->quads = !is_f64(c) && c->tune.cell_mult == 1 && ((f >= 7 && f <= 11) || (f == 3 && c->n > kGroupMax));
+    CK(c, Launch<R>::grid(c->b, c->n, (uint32_t) c->ctot, c->quads, c->stream));
     return SPH_OK;
 }
 template <class R>

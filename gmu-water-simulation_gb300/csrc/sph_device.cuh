@@ -398,11 +398,24 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
 }
 
 
-// Rank of id among the ids of its cell, the slots tmp[b, e): the number of smaller ids. Cells of
-// at most kBigCell particles are counted directly (occupancy^2 work per cell, trivial at such
-// sizes). Larger cells, up to kBigCellMax, have had their slots sorted by k_sort_big, and the
-// rank is a lower-bound search. Cells above kBigCellMax (thousands of times the rest density)
-// keep the count.
+// Rank of id among the ids of its cell, the slots tmp[b, e): the number of smaller ids, counted. In a
+// step that is cheap beside the neighbour passes even in a crowded cell: a warp's lanes mostly share the
+// cell and its loads, about 2 instructions a listed id, where the density pass spends over 300 (27 cells).
+// (A sort of the crowded cells' ids before a search was one more kernel in every step, 3 to 5 us.)
+__device__ __forceinline__ uint32_t count_rank(const uint32_t *__restrict__ tmp, uint32_t b, uint32_t e, uint32_t id)
+{
+    uint32_t r = 0, k = b;
+    for (; k + 8 <= e; k += 8) {
+#pragma unroll
+        for (uint32_t u = 0; u < 8; u++) r += tmp[k + u] < id ? 1u : 0u;
+    }
+    for (; k < e; k++) r += tmp[k] < id ? 1u : 0u;
+    return r;
+}
+
+// The same for the allocation-free grid build, where no neighbour pass follows: cells above kBigCell
+// particles, up to kBigCellMax, have had their slots sorted by k_sort_big, and the rank is a
+// lower-bound search. Cells above kBigCellMax (thousands of times the rest density) keep the count.
 __device__ __forceinline__ uint32_t rank_in_cell(const uint32_t *__restrict__ tmp, uint32_t b, uint32_t e,
                                                  uint32_t id)
 {
@@ -416,9 +429,7 @@ __device__ __forceinline__ uint32_t rank_in_cell(const uint32_t *__restrict__ tm
         }
         return lo - b;
     }
-    uint32_t r = 0;
-    for (uint32_t k = b; k < e; k++) r += tmp[k] < id ? 1u : 0u;
-    return r;
+    return count_rank(tmp, b, e, id);
 }
 
 }  // namespace sph

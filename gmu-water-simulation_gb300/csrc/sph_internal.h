@@ -45,7 +45,7 @@ struct Consts {
     float inv_cell_f;
     double cell_d;
     // particles per group of kScanTile cells of the step grid: every hash adds to it beside the
-    // cell's count, the scan reads it for its tile offsets, the crowded-cell sort clears it
+    // cell's count, the scan reads it for its tile offsets, the rank pass clears it
     uint32_t *gsum;
 };
 
@@ -60,7 +60,8 @@ struct DevBufs {
     uint32_t *count;       // particles per global cell (hash output; the slot pass counts it back to 0)
     uint32_t *start;       // exclusive scan of count, ncells_total + 1 entries
     uint32_t *bsum;        // particles per kScanTile-cell group (Consts::gsum), ncells / kScanTile + 1 words
-    uint32_t *big;         // cells above kBigCell particles: count in word 0, then the cells (big_words(n) words)
+    uint32_t *big;         // allocation-free build only (else null): cells above kBigCell particles, their number
+                           // in word 0, then the cells (big_words(n) words)
     SceneDev *scenes;
     ObstacleDev *obstacles;
     uint32_t *scene_off;   // first output index of every scene (id-order downloads)
@@ -166,11 +167,10 @@ constexpr int kMaskWordsPerParticle = 36;
 // size (plus one), enough for any tile size, and is sized with it wherever it is allocated.
 constexpr uint32_t kScanTile = 1024;
 
-// Cells holding more than kBigCell particles are listed by the scan and their slot ids sorted
-// (k_sort_big), so that the canonical rank is a search instead of an occupancy^2 count (cells up
-// to kBigCell, 16 times the rest occupancy, are counted directly: at most 128 loads a particle).
-// Sorting happens in shared memory for cells of up to kBigCellMax particles. The list holds its
-// length in word 0 and at most n / kBigCell cells: big_words(n) words.
+// In the allocation-free grid build, cells holding more than kBigCell particles are listed by the scan
+// and their slot ids sorted (k_sort_big), so that the canonical rank is a search instead of an
+// occupancy^2 count. Sorting happens in shared memory for cells of up to kBigCellMax particles. The
+// list holds its length in word 0 and at most n / kBigCell cells: big_words(n) words.
 constexpr uint32_t kBigCell = 128;
 constexpr uint32_t kBigCellMax = 4096;
 __host__ __device__ constexpr uint64_t big_words(uint64_t n) { return n / kBigCell + 2; }
@@ -184,8 +184,9 @@ struct Launch {
     static cudaError_t ingest(const DevBufs &b, const float *xyz, const float *vel, uint32_t first, uint32_t n,
                               int32_t scene, uint32_t id0, uint32_t nscenes, Consts<R> c, cudaStream_t st);
     static cudaError_t scan(const DevBufs &b, uint32_t ncells, cudaStream_t st);
+    // the grid pass: cell starts, slots, canonical order (in one launch where grid_small says so).
     // quads: also the positions as quads of four, in st_xyz (plain form)
-    static cudaError_t permute(const DevBufs &b, uint32_t n, uint32_t ncells, bool quads, cudaStream_t st);
+    static cudaError_t grid(const DevBufs &b, uint32_t n, uint32_t ncells, bool quads, cudaStream_t st);
     // positions of the first n *_u particles hashed again into the step grid (after the cell
     // multiple changed): counts and the cells of cid_u
     static cudaError_t rehash(const DevBufs &b, uint32_t n, Consts<R> c, cudaStream_t st);
@@ -201,14 +202,20 @@ struct Launch {
     static cudaError_t stats(const DevBufs &b, uint32_t nscenes, Consts<R> c, int layout_sorted, cudaStream_t st);
 };
 
-// slot assignment of the counting sort alone (the mixed form has its own permute), on a grid
-// of ncells cells
-cudaError_t launch_slot(const DevBufs &b, uint32_t n, uint32_t ncells, cudaStream_t st);
+// Scenes whose grid pass runs as one cluster of 8 blocks, a thread a particle (sph_grid_small.cuh), on
+// grids that the cluster scans in at most two tiles a block.
+constexpr int kSmallBlocks = 8, kSmallThreads = 1024;
+constexpr uint32_t kSmallParticles = kSmallBlocks * kSmallThreads, kSmallCells = 65536;
+inline bool grid_small(uint32_t n, uint32_t ncells)
+{
+    return n != 0 && n <= kSmallParticles && ncells <= kSmallCells;
+}
 
-// sorts the slot ids of every cell the scan listed in big (after the slots are taken) and
-// clears the group sums gsum of a grid of ncells cells
-cudaError_t launch_sort_big(const uint32_t *start, uint32_t *tmp, const uint32_t *big, uint32_t *gsum,
-                            uint32_t ncells, cudaStream_t st);
+// slot assignment of the counting sort alone (the mixed form has its own permute)
+cudaError_t launch_slot(const DevBufs &b, uint32_t n, cudaStream_t st);
+
+// sorts the slot ids of every cell the scan listed in big (after the slots are taken)
+cudaError_t launch_sort_big(const uint32_t *start, uint32_t *tmp, const uint32_t *big, cudaStream_t st);
 
 // disc emitter on the device (sph_emit.cu): n particles into the float3 staging arrays
 cudaError_t launch_emit_fountain(uint64_t seed, uint32_t step, uint32_t n, const float center[3], float radius,
@@ -255,7 +262,7 @@ cudaError_t group_density(const DevBufs &b, uint32_t n, Consts<double> c, cudaSt
 cudaError_t group_forces(const DevBufs &b, uint32_t n, Consts<double> c, bool record_acc, cudaStream_t st);
 
 // mixed-precision passes (sph_mixed.cu)
-cudaError_t mixed_permute(const DevBufs &b, uint32_t n, Consts<float> c, MixConsts mc, cudaStream_t st);
+cudaError_t mixed_grid(const DevBufs &b, uint32_t n, uint32_t ncells, Consts<float> c, MixConsts mc, cudaStream_t st);
 cudaError_t mixed_density(const DevBufs &b, uint32_t n, Consts<float> c, MixConsts mc, int cell_mult,
                           cudaStream_t st);
 // variant: the mixed force pass's launch form, 0..kMixedVariants-1 (all give the same bits)

@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include "sph_device.cuh"
+#include "sph_grid_small.cuh"
 #include "sph_internal.h"
 
 namespace sph {
@@ -69,7 +70,7 @@ __global__ void __launch_bounds__(256) k_ingest(Vec4<R> *__restrict__ pos_u, Vec
 // Replaces scan_local / increment_local_scans (resources/kernels/sph_grid.cl:71-121, 9-23)
 // and its sums-buffer race. The counts are left as they are: the slot pass takes every slot
 // by decrementing its cell's count, which leaves the counts at zero for the next hash; the
-// crowded-cell sort clears the group sums.
+// rank pass clears the group sums.
 // A tile is Q groups of 256 x 4 cells: each thread reads one 16-byte group of 4 counts per
 // group (coalesced across the block) and the groups are scanned one after another. Q = 1 (1024
 // cells) gives enough blocks to fill the GPU on grids of a few hundred thousand cells; grids of
@@ -157,7 +158,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const uint32_t *__r
         const uint32_t run = block_exclusive_scan(c.x + c.y + c.z + c.w, total) + off;
         off += total;
         const uint4 st4v = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
-        if (big) {  // cells above kBigCell particles get their slot ids sorted before the rank
+        if (big) {  // cells above kBigCell particles are listed (the allocation-free build sorts their slot ids)
             const uint32_t cv[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
             for (int k = 0; k < 4; k++)
@@ -223,19 +224,16 @@ __global__ void __launch_bounds__(256) k_slot(const uint2 *__restrict__ cid_u, u
     }
 }
 
-// Slot ids of the listed big cells sorted ascending in place (one block per cell at a time,
+// For the allocation-free grid build: slot ids of the listed big cells sorted ascending in place (one block per cell at a time,
 // bitonic sort in shared memory over the cell's ids padded to a power of two). Cells above
 // kBigCellMax are left as they are: rank_in_cell counts them.
 constexpr int SORT_THREADS = 256;
 
 __global__ void __launch_bounds__(SORT_THREADS) k_sort_big(const uint32_t *__restrict__ start, uint32_t *__restrict__ tmp,
-                                                           const uint32_t *__restrict__ big,
-                                                           uint32_t *__restrict__ gsum, uint32_t ngroups)
+                                                           const uint32_t *__restrict__ big)
 {
     __shared__ uint32_t sk[kBigCellMax];
     chain_wait();
-    // the scan has read the group sums: zero for the next hash
-    for (uint32_t t = blockIdx.x * SORT_THREADS + threadIdx.x; t < ngroups; t += gridDim.x * SORT_THREADS) gsum[t] = 0;
     const uint32_t nbig = big[0];
     for (uint32_t q = blockIdx.x; q < nbig; q += gridDim.x) {
         const uint32_t cell = big[1 + q];
@@ -263,39 +261,56 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_big(const uint32_t *__res
     }
 }
 
-// One particle per thread here (more per thread measured slower: the rank loop's registers cost
-// more occupancy than the overlap gains); the state loads are issued before the rank is counted.
+// What the grid pass makes of a particle: its position and velocity in sorted order, and its position
+// once more as the next passes read it: rounded to float for the FP64 form's first test of its
+// candidates, or in the quads of the plain form's density pass (k_density_quad; null: not wanted).
 template <class R>
-__global__ void __launch_bounds__(256) k_rank_permute(const uint2 *__restrict__ cid_u, uint32_t n,
+struct PlacePlain {
+    const Vec4<R> *pos_u, *vel_u;
+    Vec4<R> *pos_s, *vel_s;
+    float *posf;
+    Vec4<R> p, v;
+    __device__ __forceinline__ void fetch(uint32_t i)
+    {
+        p = ld4(pos_u + i);
+        v = ld4(vel_u + i);
+    }
+    __device__ __forceinline__ void store(uint32_t dst) const
+    {
+        st4(pos_s + dst, p);
+        st4(vel_s + dst, v);
+        if constexpr (sizeof(R) == 8) {
+            posf[3 * (size_t) dst] = (float) p.x;
+            posf[3 * (size_t) dst + 1] = (float) p.y;
+            posf[3 * (size_t) dst + 2] = (float) p.z;
+        } else if (posf) {
+            float *q = posf + 12 * (size_t) (dst >> 2) + (dst & 3u);
+            q[0] = p.x;
+            q[4] = p.y;
+            q[8] = p.z;
+        }
+    }
+};
+
+// One particle per thread here (more per thread measured slower: the rank loop's registers cost
+// more occupancy than the overlap gains); the state loads are issued before the rank is counted. It also
+// clears the group sums, which the scan has read, for the next hash.
+template <class R>
+__global__ void __launch_bounds__(256) k_rank_permute(PlacePlain<R> place, const uint2 *__restrict__ cid_u, uint32_t n,
                                                       const uint32_t *__restrict__ start,
-                                                      const uint32_t *__restrict__ tmp,
-                                                      const Vec4<R> *__restrict__ pos_u,
-                                                      const Vec4<R> *__restrict__ vel_u,
-                                                      Vec4<R> *__restrict__ pos_s, Vec4<R> *__restrict__ vel_s,
-                                                      uint32_t *__restrict__ big, float *__restrict__ posf)
+                                                      const uint32_t *__restrict__ tmp, uint32_t *__restrict__ gsum,
+                                                      uint32_t ngroups)
 {
     chain_wait();
-    if (blockIdx.x == 0 && threadIdx.x == 0) big[0] = 0;  // the crowded-cell list is used: empty for the next scan
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t t = i; t < ngroups; t += gridDim.x * blockDim.x) gsum[t] = 0;
     if (i >= n) return;
     const uint2 cd = cid_u[i];
-    const Vec4<R> p = ld4(pos_u + i), v = ld4(vel_u + i);
+    place.fetch(i);
     const uint32_t b = start[cd.x], e = start[cd.x + 1];
     if (!sph_check(b <= e && e <= n, CHK_SORT)) return;
-    const uint32_t dst = b + rank_in_cell(tmp, b, e, cd.y);
-    if (!sph_check(dst < e, CHK_SORT)) return;
-    st4(pos_s + dst, p);
-    st4(vel_s + dst, v);
-    if constexpr (sizeof(R) == 8) {  // rounded positions for the FP64 form's first test of its candidates
-        posf[3 * (size_t) dst] = (float) p.x;
-        posf[3 * (size_t) dst + 1] = (float) p.y;
-        posf[3 * (size_t) dst + 2] = (float) p.z;
-    } else if (posf) {  // quads of positions for the density pass (k_density_quad)
-        float *q = posf + 12 * (size_t) (dst >> 2) + (dst & 3u);
-        q[0] = p.x;
-        q[4] = p.y;
-        q[8] = p.z;
-    }
+    const uint32_t dst = b + count_rank(tmp, b, e, cd.y);
+    if (sph_check(dst < e, CHK_SORT)) place.store(dst);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1079,14 +1094,16 @@ cudaError_t Launch<R>::scan(const DevBufs &b, uint32_t ncells, cudaStream_t st)
 }
 
 template <class R>
-cudaError_t Launch<R>::permute(const DevBufs &b, uint32_t n, uint32_t ncells, bool quads, cudaStream_t st)
+cudaError_t Launch<R>::grid(const DevBufs &b, uint32_t n, uint32_t ncells, bool quads, cudaStream_t st)
 {
-    if (!n) return cudaSuccess;
-    cudaError_t e = launch_slot(b, n, ncells, st);
-    if (e != cudaSuccess) return e;
-    return launch_chained(k_rank_permute<R>, nblk(n, 256), 256, st, b.cid_u, n, b.start, b.tmp,
-                          (const Vec4<R> *) b.pos_u, (const Vec4<R> *) b.vel_u, (Vec4<R> *) b.pos_s,
-                          (Vec4<R> *) b.vel_s, b.big, quads || sizeof(R) == 8 ? b.st_xyz : (float *) nullptr);
+    const PlacePlain<R> place = {(const Vec4<R> *) b.pos_u, (const Vec4<R> *) b.vel_u, (Vec4<R> *) b.pos_s,
+                                 (Vec4<R> *) b.vel_s, quads || sizeof(R) == 8 ? b.st_xyz : (float *) nullptr, {}, {}};
+    if (grid_small(n, ncells)) return launch_grid_small(place, b, n, ncells, st);
+    cudaError_t e = scan(b, ncells, st);
+    if (e == cudaSuccess) e = launch_slot(b, n, st);
+    if (e != cudaSuccess || !n) return e;
+    return launch_chained(k_rank_permute<R>, nblk(n, 256), 256, st, place, b.cid_u, n, b.start, b.tmp, b.bsum,
+                          ncells / kScanTile + 1);
 }
 
 template <class R>
@@ -1248,20 +1265,16 @@ cudaError_t Launch<R>::stats(const DevBufs &b, uint32_t nscenes, Consts<R> c, in
     return cudaGetLastError();
 }
 
-cudaError_t launch_slot(const DevBufs &b, uint32_t n, uint32_t ncells, cudaStream_t st)
+cudaError_t launch_slot(const DevBufs &b, uint32_t n, cudaStream_t st)
 {
     if (!n) return cudaSuccess;
-    const cudaError_t e =
-        launch_chained(k_slot<SLOT_PER>, nblk(n, 256 * SLOT_PER), 256, st, b.cid_u, n, b.start, b.count, b.tmp);
-    return e == cudaSuccess ? launch_sort_big(b.start, b.tmp, b.big, b.bsum, ncells, st) : e;
+    return launch_chained(k_slot<SLOT_PER>, nblk(n, 256 * SLOT_PER), 256, st, b.cid_u, n, b.start, b.count, b.tmp);
 }
 
-cudaError_t launch_sort_big(const uint32_t *start, uint32_t *tmp, const uint32_t *big, uint32_t *gsum,
-                            uint32_t ncells, cudaStream_t st)
+cudaError_t launch_sort_big(const uint32_t *start, uint32_t *tmp, const uint32_t *big, cudaStream_t st)
 {
-    // a fixed grid walks the list (its length is known only on the device); with no big cell
-    // every block only clears its share of the group sums
-    return launch_chained(k_sort_big, 152, SORT_THREADS, st, start, tmp, big, gsum, ncells / kScanTile + 1);
+    // a fixed grid walks the list (its length is known only on the device)
+    return launch_chained(k_sort_big, 152, SORT_THREADS, st, start, tmp, big);
 }
 
 template struct Launch<float>;

@@ -23,6 +23,7 @@
 #include <stdint.h>
 
 #include "sph_device.cuh"
+#include "sph_grid_small.cuh"
 #include "sph_group.cuh"
 #include "sph_internal.h"
 
@@ -78,32 +79,48 @@ __device__ __forceinline__ uint4 make_record(uint2 g, float vx, float vy, float 
 }
 
 // ---- grid: canonical rank + permute, writing the master state and the gather records ----
+struct PlaceMixed {
+    const Vec4<float> *pos_u, *lo_u, *vel_u;
+    const SceneDev *scenes;
+    float h, inv_h, to_units;
+    Vec4<float> *pos_s, *lo_s, *vel_s;
+    uint2 *gpos;
+    Vec4<float> p, lo, v;
+    __device__ __forceinline__ void fetch(uint32_t i)
+    {
+        p = ld4(pos_u + i);
+        lo = ld4(lo_u + i);
+        v = ld4(vel_u + i);
+    }
+    __device__ __forceinline__ void store(uint32_t dst) const
+    {
+        st4(pos_s + dst, p);
+        st4(lo_s + dst, lo);
+        st4(vel_s + dst, v);
+        const SceneDev sc = load_scene(scenes, wbits(p.w));
+        const uint32_t qx = axis_code(p.x, lo.x, sc.half[0], h, inv_h, to_units);
+        const uint32_t qy = axis_code(p.y, lo.y, sc.half[1], h, inv_h, to_units);
+        const uint32_t qz = axis_code(p.z, lo.z, sc.half[2], h, inv_h, to_units);
+        gpos[dst] = make_uint2(qx | (qy << 16), qz);
+    }
+};
+
 // (the state loads issued before the rank is counted, as in the plain form's k_rank_permute)
-__global__ void __launch_bounds__(256) k_rank_permute_mixed(
-    const uint2 *__restrict__ cid_u, uint32_t n, const uint32_t *__restrict__ start, const uint32_t *__restrict__ tmp,
-    const Vec4<float> *__restrict__ pos_u, const Vec4<float> *__restrict__ lo_u, const Vec4<float> *__restrict__ vel_u,
-    const SceneDev *__restrict__ scenes, Consts<float> c, MixConsts mc, Vec4<float> *__restrict__ pos_s,
-    Vec4<float> *__restrict__ lo_s, Vec4<float> *__restrict__ vel_s, uint2 *__restrict__ gpos,
-    uint32_t *__restrict__ big)
+__global__ void __launch_bounds__(256) k_rank_permute_mixed(PlaceMixed place, const uint2 *__restrict__ cid_u, uint32_t n,
+                                                            const uint32_t *__restrict__ start,
+                                                            const uint32_t *__restrict__ tmp,
+                                                            uint32_t *__restrict__ gsum, uint32_t ngroups)
 {
     chain_wait();
-    if (blockIdx.x == 0 && threadIdx.x == 0) big[0] = 0;  // the crowded-cell list is used: empty for the next scan
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t t = i; t < ngroups; t += gridDim.x * blockDim.x) gsum[t] = 0;  // for the next hash
     if (i >= n) return;
     const uint2 cd = cid_u[i];
-    const Vec4<float> p = ld4(pos_u + i), lo = ld4(lo_u + i), v = ld4(vel_u + i);
+    place.fetch(i);
     const uint32_t b = start[cd.x], e = start[cd.x + 1];
     if (!sph_check(b <= e && e <= n, CHK_SORT)) return;
-    const uint32_t dst = b + rank_in_cell(tmp, b, e, cd.y);
-    if (!sph_check(dst < e, CHK_SORT)) return;
-    st4(pos_s + dst, p);
-    st4(lo_s + dst, lo);
-    st4(vel_s + dst, v);
-    const SceneDev sc = load_scene(scenes, wbits(p.w));
-    const uint32_t qx = axis_code(p.x, lo.x, sc.half[0], c.h, c.inv_h_f, mc.to_units);
-    const uint32_t qy = axis_code(p.y, lo.y, sc.half[1], c.h, c.inv_h_f, mc.to_units);
-    const uint32_t qz = axis_code(p.z, lo.z, sc.half[2], c.h, c.inv_h_f, mc.to_units);
-    gpos[dst] = make_uint2(qx | (qy << 16), qz);
+    const uint32_t dst = b + count_rank(tmp, b, e, cd.y);
+    if (sph_check(dst < e, CHK_SORT)) place.store(dst);
 }
 
 // Kahan step with explicitly rounded operations (no reassociation, no fused multiply-add)
@@ -549,13 +566,18 @@ __global__ void __launch_bounds__(256) k_egress_mixed(const Vec4<float> *__restr
 // ---- launchers ----------------------------------------------------------------------------
 static inline unsigned nblk(uint32_t n, unsigned t) { return (unsigned) ((n + t - 1) / t); }
 
-cudaError_t mixed_permute(const DevBufs &b, uint32_t n, Consts<float> c, MixConsts mc, cudaStream_t st)
+cudaError_t mixed_grid(const DevBufs &b, uint32_t n, uint32_t ncells, Consts<float> c, MixConsts mc, cudaStream_t st)
 {
-    if (!n) return cudaSuccess;
-    return launch_chained(k_rank_permute_mixed, nblk(n, 256), 256, st, b.cid_u, n, b.start, b.tmp,
-                          (const Vec4<float> *) b.pos_u, (const Vec4<float> *) b.lo_u, (const Vec4<float> *) b.vel_u,
-                          b.scenes, c, mc, (Vec4<float> *) b.pos_s, (Vec4<float> *) b.lo_s, (Vec4<float> *) b.vel_s,
-                          b.gpos, b.big);
+    const PlaceMixed place = {(const Vec4<float> *) b.pos_u, (const Vec4<float> *) b.lo_u,
+                              (const Vec4<float> *) b.vel_u, b.scenes, c.h, c.inv_h_f, mc.to_units,
+                              (Vec4<float> *) b.pos_s, (Vec4<float> *) b.lo_s, (Vec4<float> *) b.vel_s, b.gpos,
+                              {}, {}, {}};
+    if (grid_small(n, ncells)) return launch_grid_small(place, b, n, ncells, st);
+    cudaError_t e = Launch<float>::scan(b, ncells, st);
+    if (e == cudaSuccess) e = launch_slot(b, n, st);
+    if (e != cudaSuccess || !n) return e;
+    return launch_chained(k_rank_permute_mixed, nblk(n, 256), 256, st, place, b.cid_u, n, b.start, b.tmp, b.bsum,
+                          ncells / kScanTile + 1);
 }
 
 // Where the group forms are used: as for the plain form (group_density). Density and forces together, in

@@ -142,7 +142,7 @@ cudaError_t ref_grid_build(const float *xyz, uint32_t n, int3 res, float3 half, 
     e = Launch<float>::scan(b, (uint32_t) ncells, st);  // starts
     if (e == cudaSuccess && n) {
         k_slot_ids<<<blocks, 256, 0, st>>>(out_cell, n, b.start, out_order, b.tmp);
-        e = launch_sort_big(b.start, b.tmp, b.big, b.bsum, (uint32_t) ncells, st);
+        e = launch_sort_big(b.start, b.tmp, b.big, st);
         if (e == cudaSuccess) {
             k_rank_ids<<<blocks, 256, 0, st>>>(out_cell, n, b.start, b.tmp, out_order);
             e = cudaGetLastError();
