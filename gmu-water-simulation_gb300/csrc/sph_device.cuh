@@ -413,23 +413,4 @@ __device__ __forceinline__ uint32_t count_rank(const uint32_t *__restrict__ tmp,
     return r;
 }
 
-// The same for the allocation-free grid build, where no neighbour pass follows: cells above kBigCell
-// particles, up to kBigCellMax, have had their slots sorted by k_sort_big, and the rank is a
-// lower-bound search. Cells above kBigCellMax (thousands of times the rest density) keep the count.
-__device__ __forceinline__ uint32_t rank_in_cell(const uint32_t *__restrict__ tmp, uint32_t b, uint32_t e,
-                                                 uint32_t id)
-{
-    const uint32_t occ = e - b;
-    if (occ > kBigCell && occ <= kBigCellMax) {
-        uint32_t lo = b, hi = e;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (tmp[mid] < id) lo = mid + 1;
-            else hi = mid;
-        }
-        return lo - b;
-    }
-    return count_rank(tmp, b, e, id);
-}
-
 }  // namespace sph

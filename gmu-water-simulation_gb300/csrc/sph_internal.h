@@ -168,10 +168,9 @@ constexpr int kMaskWordsPerParticle = 36;
 constexpr uint32_t kScanTile = 1024;
 
 // In the allocation-free grid build, cells holding more than kBigCell particles are listed by the scan
-// and their slot ids sorted (k_sort_big), so that the canonical rank is a search instead of an
-// occupancy^2 count. Sorting happens in shared memory for cells of up to kBigCellMax particles. The
+// and ordered by a whole block (k_order_cells), in shared memory up to kBigCellMax particles. The
 // list holds its length in word 0 and at most n / kBigCell cells: big_words(n) words.
-constexpr uint32_t kBigCell = 128;
+constexpr uint32_t kBigCell = 32;
 constexpr uint32_t kBigCellMax = 4096;
 __host__ __device__ constexpr uint64_t big_words(uint64_t n) { return n / kBigCell + 2; }
 
@@ -213,9 +212,6 @@ inline bool grid_small(uint32_t n, uint32_t ncells)
 
 // slot assignment of the counting sort alone (the mixed form has its own permute)
 cudaError_t launch_slot(const DevBufs &b, uint32_t n, cudaStream_t st);
-
-// sorts the slot ids of every cell the scan listed in big (after the slots are taken)
-cudaError_t launch_sort_big(const uint32_t *start, uint32_t *tmp, const uint32_t *big, cudaStream_t st);
 
 // disc emitter on the device (sph_emit.cu): n particles into the float3 staging arrays
 cudaError_t launch_emit_fountain(uint64_t seed, uint32_t step, uint32_t n, const float center[3], float radius,

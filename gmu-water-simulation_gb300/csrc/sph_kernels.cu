@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const uint32_t *__r
         const uint32_t run = block_exclusive_scan(c.x + c.y + c.z + c.w, total) + off;
         off += total;
         const uint4 st4v = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
-        if (big) {  // cells above kBigCell particles are listed (the allocation-free build sorts their slot ids)
+        if (big) {  // cells above kBigCell particles are listed (for the allocation-free build)
             const uint32_t cv[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
             for (int k = 0; k < 4; k++)
@@ -221,43 +221,6 @@ __global__ void __launch_bounds__(256) k_slot(const uint2 *__restrict__ cid_u, u
                                           __ffs(peers[k]) - 1);
         const uint32_t t = base + (uint32_t) __popc(peers[k] & ((1u << lane) - 1u));
         if (cd[k].x != kNoCell && sph_check(t < n, CHK_SORT)) tmp[t] = cd[k].y;
-    }
-}
-
-// For the allocation-free grid build: slot ids of the listed big cells sorted ascending in place (one block per cell at a time,
-// bitonic sort in shared memory over the cell's ids padded to a power of two). Cells above
-// kBigCellMax are left as they are: rank_in_cell counts them.
-constexpr int SORT_THREADS = 256;
-
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_big(const uint32_t *__restrict__ start, uint32_t *__restrict__ tmp,
-                                                           const uint32_t *__restrict__ big)
-{
-    __shared__ uint32_t sk[kBigCellMax];
-    chain_wait();
-    const uint32_t nbig = big[0];
-    for (uint32_t q = blockIdx.x; q < nbig; q += gridDim.x) {
-        const uint32_t cell = big[1 + q];
-        const uint32_t b = start[cell], e = start[cell + 1], occ = e - b;
-        if (occ <= kBigCell || occ > kBigCellMax) continue;
-        uint32_t P = 2 * kBigCell;
-        while (P < occ) P <<= 1;
-        for (uint32_t t = threadIdx.x; t < P; t += SORT_THREADS) sk[t] = t < occ ? tmp[b + t] : 0xffffffffu;
-        __syncthreads();
-        for (uint32_t k = 2; k <= P; k <<= 1) {
-            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                for (uint32_t t = threadIdx.x; t < P / 2; t += SORT_THREADS) {
-                    const uint32_t lo = 2 * j * (t / j) + (t % j), hi = lo + j;  // lo has bit j clear
-                    const uint32_t x = sk[lo], y = sk[hi];
-                    if ((x > y) == ((lo & k) == 0)) {
-                        sk[lo] = y;
-                        sk[hi] = x;
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        for (uint32_t t = threadIdx.x; t < occ; t += SORT_THREADS) tmp[b + t] = sk[t];
-        __syncthreads();
     }
 }
 
@@ -1269,12 +1232,6 @@ cudaError_t launch_slot(const DevBufs &b, uint32_t n, cudaStream_t st)
 {
     if (!n) return cudaSuccess;
     return launch_chained(k_slot<SLOT_PER>, nblk(n, 256 * SLOT_PER), 256, st, b.cid_u, n, b.start, b.count, b.tmp);
-}
-
-cudaError_t launch_sort_big(const uint32_t *start, uint32_t *tmp, const uint32_t *big, cudaStream_t st)
-{
-    // a fixed grid walks the list (its length is known only on the device)
-    return launch_chained(k_sort_big, 152, SORT_THREADS, st, start, tmp, big);
 }
 
 template struct Launch<float>;

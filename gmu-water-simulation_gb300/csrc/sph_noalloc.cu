@@ -52,9 +52,10 @@ std::mutex g_scratch_mu;
 __global__ void __launch_bounds__(256) k_hash_plain_xyz(const float *__restrict__ xyz, uint32_t n, float3 half,
                                                         int3 res, float inv_h, double h_d,
                                                         uint32_t *__restrict__ out_cell, uint32_t *__restrict__ count,
-                                                        uint32_t *__restrict__ slot)
+                                                        uint32_t *__restrict__ slot, uint32_t *__restrict__ big)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) big[0] = 0;  // the crowded-cell list, for the scan
     if (i >= n) return;
     const int cx = cell_axis(xyz[3 * i], half.x, inv_h, h_d, res.x);
     const int cy = cell_axis(xyz[3 * i + 1], half.y, inv_h, h_d, res.y);
@@ -69,11 +70,12 @@ __global__ void __launch_bounds__(256) k_hash_plain_xyz(const float *__restrict_
     slot[i] = __shfl_sync(act, first, lead) + (uint32_t) __popc(peers & ((1u << lane) - 1u));
 }
 
-// particles of each group of kScanTile cells, for the scan's tile offsets, and the crowded-cell list
-// emptied for it (one block a group: 4 coalesced loads a thread)
+// particles of each group of kScanTile cells, for the scan's tile offsets (one block a group: 4 coalesced
+// loads a thread)
 __global__ void __launch_bounds__(256) k_group_sums(const uint32_t *__restrict__ count, uint32_t ncells,
-                                                    uint32_t *__restrict__ gsum, uint32_t *__restrict__ big)
+                                                    uint32_t *__restrict__ gsum)
 {
+    chain_wait();
     static_assert(kScanTile == 4 * 256, "four cells a thread");
     __shared__ uint32_t part[8];
     uint32_t v = 0;
@@ -89,7 +91,6 @@ __global__ void __launch_bounds__(256) k_group_sums(const uint32_t *__restrict__
         uint32_t t = 0;
         for (int w = 0; w < 8; w++) t += part[w];
         gsum[blockIdx.x] = t;
-        if (blockIdx.x == 0) big[0] = 0;
     }
 }
 
@@ -98,21 +99,84 @@ __global__ void __launch_bounds__(256) k_slot_ids(const uint32_t *__restrict__ c
                                                   const uint32_t *__restrict__ start,
                                                   const uint32_t *__restrict__ slot, uint32_t *__restrict__ slot_ids)
 {
+    chain_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     slot_ids[start[cell[i]] + slot[i]] = i;
 }
 
-// canonical (cell, id) order: position = cell start + number of same-cell ids below i
+// Canonical (cell, id) order: position = cell start + number of same-cell ids below i, counted. A thread a
+// particle: up to kRankByParticle particles, where even a single cell of them all is a few million
+// loads; beyond, k_order_cells.
+constexpr uint32_t kRankByParticle = 65536;
+
 __global__ void __launch_bounds__(256) k_rank_ids(const uint32_t *__restrict__ cell, uint32_t n,
                                                   const uint32_t *__restrict__ start,
                                                   const uint32_t *__restrict__ slot_ids, uint32_t *__restrict__ order)
 {
+    chain_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t c = cell[i], b = start[c], e = start[c + 1];
-    const uint32_t dst = b + rank_in_cell(slot_ids, b, e, i);
+    const uint32_t dst = b + count_rank(slot_ids, b, e, i);
     if (sph_check(dst < e && e <= n, CHK_SORT)) order[dst] = i;
+}
+
+// The same by cells, a thread a cell, so that neighbouring threads read and write neighbouring slots (a
+// thread a particle reads two cell starts and the slots of a random cell). Cells above kBigCell particles
+// are left to the list: those of up to kBigCellMax sorted by one block each (bitonic, in shared memory),
+// larger ones (thousands of times the rest density) counted by all blocks together. The whole build of
+// scattered particles, with this pass and with k_rank_ids: 65,000 22.6 / 18.2 us, 520,000 34.8 / 32.8,
+// 1,040,000 46.5 / 49.2, and k_rank_ids would need a sort of crowded cells before it (3 us) at such sizes.
+__global__ void __launch_bounds__(256) k_order_cells(const uint32_t *__restrict__ start, uint32_t ncells,
+                                                     const uint32_t *__restrict__ slot_ids,
+                                                     const uint32_t *__restrict__ big, uint32_t n,
+                                                     uint32_t *__restrict__ order)
+{
+    __shared__ uint32_t sk[kBigCellMax];
+    chain_wait();
+    const uint32_t c = blockIdx.x * 256u + threadIdx.x;
+    if (c < ncells) {
+        const uint32_t b = start[c], e = start[c + 1];
+        if (sph_check(b <= e && e <= n, CHK_SORT) && e - b <= kBigCell)
+            for (uint32_t k = b; k < e; k++) {
+                const uint32_t id = slot_ids[k];
+                uint32_t r = b;
+                for (uint32_t m = b; m < e; m++) r += slot_ids[m] < id ? 1u : 0u;
+                order[r] = id;
+            }
+    }
+    const uint32_t nbig = big[0];
+    for (uint32_t q = 0; q < nbig; q++) {
+        const uint32_t cell = big[1 + q];
+        const uint32_t b = start[cell], e = start[cell + 1], occ = e - b;
+        if (!sph_check(b <= e && e <= n, CHK_SORT)) continue;
+        if (occ > kBigCellMax) {
+            for (uint32_t k = b + c; k < e; k += gridDim.x * 256u)
+                order[b + count_rank(slot_ids, b, e, slot_ids[k])] = slot_ids[k];
+            continue;
+        }
+        if (q % gridDim.x != blockIdx.x) continue;
+        uint32_t P = 2 * kBigCell;
+        while (P < occ) P <<= 1;
+        for (uint32_t t = threadIdx.x; t < P; t += 256) sk[t] = t < occ ? slot_ids[b + t] : 0xffffffffu;
+        __syncthreads();
+        for (uint32_t k = 2; k <= P; k <<= 1) {
+            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                for (uint32_t t = threadIdx.x; t < P / 2; t += 256) {
+                    const uint32_t lo = 2 * j * (t / j) + (t % j), hi = lo + j;  // lo has bit j clear
+                    const uint32_t x = sk[lo], y = sk[hi];
+                    if ((x > y) == ((lo & k) == 0)) {
+                        sk[lo] = y;
+                        sk[hi] = x;
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        for (uint32_t t = threadIdx.x; t < occ; t += 256) order[b + t] = sk[t];
+        __syncthreads();
+    }
 }
 
 }  // namespace
@@ -137,17 +201,19 @@ cudaError_t ref_grid_build(const float *xyz, uint32_t n, int3 res, float3 half, 
     const unsigned blocks = (unsigned) ((n + 255) / 256);
     // the slots wait in out_order, which only the last pass writes
     if (n)
-        k_hash_plain_xyz<<<blocks, 256, 0, st>>>(xyz, n, half, res, 1.0f / h, (double) h, out_cell, b.count, out_order);
-    k_group_sums<<<(unsigned) (ncells / kScanTile + 1), 256, 0, st>>>(b.count, (uint32_t) ncells, b.bsum, b.big);
-    e = Launch<float>::scan(b, (uint32_t) ncells, st);  // starts
-    if (e == cudaSuccess && n) {
-        k_slot_ids<<<blocks, 256, 0, st>>>(out_cell, n, b.start, out_order, b.tmp);
-        e = launch_sort_big(b.start, b.tmp, b.big, st);
-        if (e == cudaSuccess) {
-            k_rank_ids<<<blocks, 256, 0, st>>>(out_cell, n, b.start, b.tmp, out_order);
-            e = cudaGetLastError();
-        }
-    }
+        k_hash_plain_xyz<<<blocks, 256, 0, st>>>(xyz, n, half, res, 1.0f / h, (double) h, out_cell, b.count, out_order,
+                                                 b.big);
+    e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = launch_chained(k_group_sums, (unsigned) (ncells / kScanTile + 1), 256, st, b.count, (uint32_t) ncells, b.bsum);
+    if (e == cudaSuccess) e = Launch<float>::scan(b, (uint32_t) ncells, st);  // starts
+    if (e == cudaSuccess && n)
+        e = launch_chained(k_slot_ids, blocks, 256, st, out_cell, n, out_start, out_order, b.tmp);
+    if (e == cudaSuccess && n)
+        e = n <= kRankByParticle
+                ? launch_chained(k_rank_ids, blocks, 256, st, out_cell, n, out_start, b.tmp, out_order)
+                : launch_chained(k_order_cells, (unsigned) ((ncells + 255) / 256), 256, st, out_start, (uint32_t) ncells,
+                                 b.tmp, b.big, n, out_order);
     return e;
 }
 
