@@ -548,17 +548,26 @@ __global__ void __launch_bounds__(256) k_egress_mixed(const Vec4<float> *__restr
         xyz[3 * o + 2] = (T) pp.z + (T) ll.z;
         v[3 * o] = vv.x; v[3 * o + 1] = vv.y; v[3 * o + 2] = vv.z;
     }
-    if (i < n_aux) {
+    // particles without a density (or an acceleration) yet, appended since, have 0 there
+    if (rho && i < n_state) {
         const Vec4<float> pp = ldc4(posA + i), vv = ldc4(velA + i);
         const uint32_t o = __ldg(scene_off + wbits(pp.w)) + wbits(vv.w);
-        const Vec4<float> ax = ldc4(aux + i);
-        rho[o] = ax.x;
-        p[o] = ax.y;
+        if (!sph_check(o < n_state, CHK_EGRESS)) return;
+        T r = 0, q = 0;
+        if (i < n_aux) {
+            const Vec4<float> ax = ldc4(aux + i);
+            r = ax.x;
+            q = ax.y;
+        }
+        rho[o] = r;
+        p[o] = q;
     }
-    if (acc && i < n_acc) {
+    if (acc && i < n_state) {
         const Vec4<float> pp = ldc4(pos_u + i), vv = ldc4(vel_u + i);
         const uint32_t o = __ldg(scene_off + wbits(pp.w)) + wbits(vv.w);
-        const Vec4<float> aa = ldc4(acc + i);
+        if (!sph_check(o < n_state, CHK_EGRESS)) return;
+        Vec4<float> aa = {0, 0, 0, 0};
+        if (i < n_acc) aa = ldc4(acc + i);
         a[3 * o] = aa.x; a[3 * o + 1] = aa.y; a[3 * o + 2] = aa.z;
     }
 }
