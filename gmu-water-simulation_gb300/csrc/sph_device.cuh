@@ -179,6 +179,14 @@ __device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf
 __device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float inv_sqrt(float x) { return rsqrtf(x); }
 __device__ __forceinline__ double inv_sqrt(double x) { return 1.0 / sqrt(x); }
+// For x that is normal (or zero, infinite, NaN): the hardware's approximation by itself, without the scaling
+// of denormal arguments that rsqrtf surrounds it with; the same value for every normal x.
+__device__ __forceinline__ float inv_sqrt_normal(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 
 // The cell of a position in the step grid (cells h / cell multiple wide), and its global index.
 template <class R>
