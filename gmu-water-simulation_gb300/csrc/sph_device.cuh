@@ -224,6 +224,17 @@ __device__ __forceinline__ R h2_minus_r2(R dx, R dy, R dz, R h2)
     t = rfma(-dy, dy, t);
     return rfma(-dz, dz, t);
 }
+// its negative, with the same roundings; an exact zero is +0 here too
+template <class R>
+__device__ __forceinline__ R r2_minus_h2(R dx, R dy, R dz, R h2)
+{
+    R t = rfma(dx, dx, -h2);
+    t = rfma(dy, dy, t);
+    return rfma(dz, dz, t);
+}
+// the sign bit of u in bit 31
+__device__ __forceinline__ uint32_t sign_word(float u) { return __float_as_uint(u); }
+__device__ __forceinline__ uint32_t sign_word(double u) { return (uint32_t) __double2hiint(u); }
 // acc + max(t, 0)^3
 template <class R>
 __device__ __forceinline__ R poly6_acc(R acc, R t)

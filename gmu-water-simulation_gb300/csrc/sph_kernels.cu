@@ -451,23 +451,24 @@ __global__ void __launch_bounds__(256) k_density_mask(const Vec4<R> *__restrict_
             if (!sph_check(jb <= je && je <= n, CHK_ROW)) continue;
             int w = 0;
             for (uint32_t cb = jb; cb < je; cb += 32, w++) {
-                // bit k of the chunk's word = candidate cb + k; bits enter at the top and
-                // move down one place per candidate
+                // bit k of the chunk's word = candidate cb + k; the sign bits of r^2 - h^2 enter at the
+                // bottom, one funnel shift each, and the word is turned round at the end
                 const uint32_t ce = min(je, cb + 32u);
                 uint32_t m = 0;
 #pragma unroll 4
                 for (uint32_t j = cb; j < ce; j++) {
                     const Vec4<R> pj = ld4(pos + j);
-                    const R t = h2_minus_r2<R>(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z, h2);
-                    m = (m >> 1) | (t > (R) 0 ? 0x80000000u : 0u);
-                    acc = poly6_acc<R>(acc, t);
+                    R u = r2_minus_h2<R>(pi.x - pj.x, pi.y - pj.y, pi.z - pj.z, h2);
+                    m = __funnelshift_l(sign_word(u), m, 1);
+                    u = u < (R) 0 ? u : (R) 0;
+                    acc = rfma(rmul(u, u), u, acc);  // minus the sum of max(h^2 - r^2, 0)^3
                 }
-                m >>= 32 - (ce - cb);
+                m = __brev(m) >> (32 - (ce - cb));
                 if (w < St::WORDS) st_keep(masks + (size_t) (r * St::WORDS + w) * n + i, m, keep);
             }
         }
     }
-    const R rho = rmul(rmul(acc, c.c_poly6), c.mass);
+    const R rho = rmul(rmul(-acc, c.c_poly6), c.mass);
     const R p = rmul(c.k, rsub(rho, c.rho0));
     const Vec4<R> ar = aux_record<R>(rho, p, c);
     const R q = ar.z, inv = ar.w;
