@@ -232,9 +232,9 @@ __device__ __forceinline__ R r2_minus_h2(R dx, R dy, R dz, R h2)
     t = rfma(dy, dy, t);
     return rfma(dz, dz, t);
 }
-// the sign bit of u in bit 31
+// bit 31 set for u < 0 (u the result of arithmetic: a float NaN then has no sign, a double NaN may have)
 __device__ __forceinline__ uint32_t sign_word(float u) { return __float_as_uint(u); }
-__device__ __forceinline__ uint32_t sign_word(double u) { return (uint32_t) __double2hiint(u); }
+__device__ __forceinline__ uint32_t sign_word(double u) { return u < 0.0 ? 0x80000000u : 0u; }
 // acc + max(t, 0)^3
 template <class R>
 __device__ __forceinline__ R poly6_acc(R acc, R t)
