@@ -419,8 +419,12 @@ __global__ void __launch_bounds__(BLOCK) k_forces_list(
 // WORDS chunks are not recorded: the force pass tests them itself. RAD = 1 is the reference's
 // 27 cells of size h; RAD = 2 walks 125 cells of size h/2 (42% less volume than 27 h^3).
 
+// Cells of h/2 (RAD 2): short rows, many of them; 75% of the issue slots and 69% of the load path used at
+// 1,000,000 fallen particles, the rest waiting for loads. At 32 registers (8 blocks an SM, a few spills) rather
+// than 48: 4,000,000 fallen 848 to 815 us, 1,000,000 at rest 137 to 133, fallen 223 to 227 alone, but a whole
+// two-step call of the latter beside others 1070 to 1058.
 template <class R, bool REC, int RAD = 1>
-__global__ void __launch_bounds__(256) k_density_mask(const Vec4<R> *__restrict__ pos, Vec4<R> *__restrict__ aux,
+__global__ void __launch_bounds__(256, RAD == 2 ? 8 : 1) k_density_mask(const Vec4<R> *__restrict__ pos, Vec4<R> *__restrict__ aux,
                                                       const uint32_t *__restrict__ start,
                                                       const SceneDev *__restrict__ scenes, uint32_t n, Consts<R> c,
                                                       uint32_t *__restrict__ masks, const Vec4<R> *__restrict__ vel,
