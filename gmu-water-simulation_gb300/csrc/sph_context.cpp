@@ -932,17 +932,18 @@ int sph_upload(sph_ctx *c, const float *xyz, const float *vel, const uint32_t *c
             // pinned caller arrays are read by the ingest kernel itself; others go through staging
             const float *sx = (const float *) pinned_view(xyz);
             const float *sv = vel ? (const float *) pinned_view(vel) : nullptr;
-            if (!sx || (vel && !sv)) {
+            const bool link = sx && (!vel || sv);
+            if (!link) {
                 CK(c, cudaMemcpyAsync(c->b.st_xyz, xyz, 12 * total, cudaMemcpyHostToDevice, c->stream));
                 if (vel) CK(c, cudaMemcpyAsync(c->b.st_vel, vel, 12 * total, cudaMemcpyHostToDevice, c->stream));
                 sx = c->b.st_xyz;
                 sv = vel ? c->b.st_vel : nullptr;
             }
             if (is_f64(c))
-                CK(c, Launch<double>::ingest(c->b, sx, sv, 0, c->n, -1, 0, (uint32_t) c->sc.size(),
+                CK(c, Launch<double>::ingest(c->b, sx, sv, link, 0, c->n, -1, 0, (uint32_t) c->sc.size(),
                                              make_consts<double>(c, c->tune.cell_mult), c->stream));
             else
-                CK(c, Launch<float>::ingest(c->b, sx, sv, 0, c->n, -1, 0, (uint32_t) c->sc.size(),
+                CK(c, Launch<float>::ingest(c->b, sx, sv, link, 0, c->n, -1, 0, (uint32_t) c->sc.size(),
                                             make_consts<float>(c, c->tune.cell_mult), c->stream));
         }
         c->state = HASHED;
@@ -976,10 +977,10 @@ int append_ingest(sph_ctx *c, uint32_t scene, uint32_t n, bool has_vel)
     SceneHost &h = c->sc[scene];
     if (is_mixed(c)) CK(c, cudaMemsetAsync((char *) c->b.lo_u + 16ull * c->n, 0, 16ull * n, c->stream));
     if (is_f64(c))
-        CK(c, Launch<double>::ingest(c->b, c->b.st_xyz, has_vel ? c->b.st_vel : nullptr, c->n, n, (int32_t) scene,
+        CK(c, Launch<double>::ingest(c->b, c->b.st_xyz, has_vel ? c->b.st_vel : nullptr, false, c->n, n, (int32_t) scene,
                                      h.count, (uint32_t) c->sc.size(), make_consts<double>(c, c->tune.cell_mult), c->stream));
     else
-        CK(c, Launch<float>::ingest(c->b, c->b.st_xyz, has_vel ? c->b.st_vel : nullptr, c->n, n, (int32_t) scene,
+        CK(c, Launch<float>::ingest(c->b, c->b.st_xyz, has_vel ? c->b.st_vel : nullptr, false, c->n, n, (int32_t) scene,
                                     h.count, (uint32_t) c->sc.size(), make_consts<float>(c, c->tune.cell_mult), c->stream));
     h.count += n;
     c->n += n;

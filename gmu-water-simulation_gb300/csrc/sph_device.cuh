@@ -69,6 +69,27 @@ inline cudaError_t launch_chained(void (*kernel)(K...), unsigned grid, unsigned 
     return cudaLaunchKernelEx(&cfg, kernel, ((K) args)...);
 }
 
+// An ordinary launch at a raised priority, for the short kernels at both ends of a call that wait for the host link
+// or for memory (ingest, handoff): with several contexts in flight their blocks go ahead of the waiting blocks
+// of another context's neighbour pass, and the transfers run beside it. At equal priorities they queue behind
+// it, until every context waits for the link at once. (The grid pass's kernels at this priority gain nothing,
+// and undo the gain at 4,000,000 particles.)
+template <typename... K, typename... A>
+inline cudaError_t launch_first(void (*kernel)(K...), unsigned grid, unsigned block, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributePriority;
+    at[0].val.priority = -1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, ((K) args)...);
+}
+
 template <class R>
 struct alignas(4 * sizeof(R)) Vec4 {
     R x, y, z, w;

@@ -32,8 +32,7 @@ cudaError_t launch_handoff(const DevBufs &b, uint32_t n, int layout_sorted, floa
     if (!n) return cudaSuccess;
     const Vec4<R> *pos = (const Vec4<R> *) (layout_sorted ? b.pos_s : b.pos_u);
     const Vec4<R> *vel = (const Vec4<R> *) (layout_sorted ? b.vel_s : b.vel_u);
-    k_handoff<R><<<(n + 255) / 256, 256, 0, st>>>(pos, vel, b.scene_off, n, xyz, v);
-    return cudaGetLastError();
+    return launch_first(k_handoff<R>, (n + 255) / 256, 256, st, pos, vel, b.scene_off, n, xyz, v);
 }
 
 // Orthographic point splat of one scene along axis `a` onto a width x height image over the

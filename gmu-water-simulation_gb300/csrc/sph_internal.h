@@ -180,8 +180,10 @@ struct Launch {
     // xyz / vel: device staging arrays of n particles stored at [first, first + n).
     // scene >= 0: all belong to that scene with ids id0..; scene < 0: scene and id follow
     // the scene_off table (upload of every scene at once, first == 0).
-    static cudaError_t ingest(const DevBufs &b, const float *xyz, const float *vel, uint32_t first, uint32_t n,
-                              int32_t scene, uint32_t id0, uint32_t nscenes, Consts<R> c, cudaStream_t st);
+    // link: the arrays are pinned host memory, read over the host link.
+    static cudaError_t ingest(const DevBufs &b, const float *xyz, const float *vel, bool link, uint32_t first,
+                              uint32_t n, int32_t scene, uint32_t id0, uint32_t nscenes, Consts<R> c,
+                              cudaStream_t st);
     static cudaError_t scan(const DevBufs &b, uint32_t ncells, cudaStream_t st);
     // the grid pass: cell starts, slots, canonical order (in one launch where grid_small says so).
     // quads: also the positions as quads of four, in st_xyz (plain form)

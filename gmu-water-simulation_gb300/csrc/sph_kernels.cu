@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "sph_device.cuh"
 #include "sph_grid_small.cuh"
 #include "sph_internal.h"
@@ -30,37 +32,46 @@ __global__ void __launch_bounds__(256) k_ingest(Vec4<R> *__restrict__ pos_u, Vec
                                                 uint32_t first, uint32_t n, int32_t fixed_scene, uint32_t id0,
                                                 Consts<R> c)
 {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    uint32_t s, id;
-    if (fixed_scene >= 0) {
-        s = (uint32_t) fixed_scene;
-        id = id0 + k;
-    } else {
-        uint32_t lo = 0, hi = nscenes;  // largest s with scene_off[s] <= k
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(scene_off + mid) <= k) lo = mid;
-            else hi = mid;
+    const uint32_t step = gridDim.x * blockDim.x;
+    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    float px = 0, py = 0, pz = 0, ux = 0, uy = 0, uz = 0;
+    auto load = [&](uint32_t j) {
+        if (j >= n) return;
+        px = xyz[3 * (size_t) j];
+        py = xyz[3 * (size_t) j + 1];
+        pz = xyz[3 * (size_t) j + 2];
+        if (!vel) return;
+        ux = vel[3 * (size_t) j];
+        uy = vel[3 * (size_t) j + 1];
+        uz = vel[3 * (size_t) j + 2];
+    };
+    load(k);
+    for (; k < n; k += step) {
+        const R x = (R) px, y = (R) py, z = (R) pz, vx = (R) ux, vy = (R) uy, vz = (R) uz;
+        load(k + step);
+        uint32_t s, id;
+        if (fixed_scene >= 0) {
+            s = (uint32_t) fixed_scene;
+            id = id0 + k;
+        } else {
+            uint32_t lo = 0, hi = nscenes;  // largest s with scene_off[s] <= k
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (__ldg(scene_off + mid) <= k) lo = mid;
+                else hi = mid;
+            }
+            s = lo;
+            id = k - __ldg(scene_off + s);
         }
-        s = lo;
-        id = k - __ldg(scene_off + s);
+        const SceneDev sc = load_scene(scenes, s);
+        int cx, cy, cz;
+        const uint32_t cell = hash_cell<R>(sc, x, y, z, c, cx, cy, cz);
+        count_add(count, c.gsum, cell);
+        const uint32_t i = first + k;
+        st4(pos_u + i, Vec4<R>{x, y, z, mkw<R>(s)});
+        st4(vel_u + i, Vec4<R>{vx, vy, vz, mkw<R>(id)});
+        cid_u[i] = make_uint2(cell, id);
     }
-    const SceneDev sc = load_scene(scenes, s);
-    const R x = (R) xyz[3 * k], y = (R) xyz[3 * k + 1], z = (R) xyz[3 * k + 2];
-    R vx = 0, vy = 0, vz = 0;
-    if (vel) {
-        vx = (R) vel[3 * k];
-        vy = (R) vel[3 * k + 1];
-        vz = (R) vel[3 * k + 2];
-    }
-    int cx, cy, cz;
-    const uint32_t cell = hash_cell<R>(sc, x, y, z, c, cx, cy, cz);
-    count_add(count, c.gsum, cell);
-    const uint32_t i = first + k;
-    st4(pos_u + i, Vec4<R>{x, y, z, mkw<R>(s)});
-    st4(vel_u + i, Vec4<R>{vx, vy, vz, mkw<R>(id)});
-    cid_u[i] = make_uint2(cell, id);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1047,14 +1058,22 @@ __global__ void k_stats_final(const double *__restrict__ partial, const uint32_t
 // ------------------------------------------------------------------------------------
 static inline unsigned nblk(uint32_t n, unsigned t) { return (unsigned) ((n + t - 1) / t); }
 
+// Blocks of an ingest that reads pinned host memory. 96 blocks, each thread with the next particle's loads in
+// flight, keep the link busy (a call alone takes as long as with every block resident), and leave the SMs to
+// other contexts' passes. Time per call, three contexts in turn, with every block at the ordinary priority / 96
+// blocks at the raised one: two steps of 1,000,000 at rest 559 / 511 us, fallen (cells of h/2) 1060 / 981, a
+// batch of 48 scenes 658 / 590, one step of 4,000,000 2352 / 2020. Alone: 627 / 629, 1200 / 1201, 773 / 773,
+// 2445 / 2449. 152 blocks: 513, 999, 597, 2106 in turn; 76: 511, 978, 590, 1995 in turn but 644 alone at rest.
+constexpr unsigned kLinkBlocks = 96;
+
 template <class R>
-cudaError_t Launch<R>::ingest(const DevBufs &b, const float *xyz, const float *vel, uint32_t first, uint32_t n,
-                              int32_t scene, uint32_t id0, uint32_t nscenes, Consts<R> c, cudaStream_t st)
+cudaError_t Launch<R>::ingest(const DevBufs &b, const float *xyz, const float *vel, bool link, uint32_t first,
+                              uint32_t n, int32_t scene, uint32_t id0, uint32_t nscenes, Consts<R> c, cudaStream_t st)
 {
     if (!n) return cudaSuccess;
-    k_ingest<R><<<nblk(n, 256), 256, 0, st>>>((Vec4<R> *) b.pos_u, (Vec4<R> *) b.vel_u, b.cid_u, b.count, b.scenes,
-                                              b.scene_off, nscenes, xyz, vel, first, n, scene, id0, c);
-    return cudaGetLastError();
+    const unsigned most = link ? kLinkBlocks : 0xffffffffu;
+    return launch_first(k_ingest<R>, std::min(nblk(n, 256), most), 256, st, (Vec4<R> *) b.pos_u, (Vec4<R> *) b.vel_u,
+                        b.cid_u, b.count, b.scenes, b.scene_off, nscenes, xyz, vel, first, n, scene, id0, c);
 }
 
 template <class R>
