@@ -1244,11 +1244,9 @@ cudaError_t Launch<R>::egress(const DevBufs &b, uint32_t n_state, uint32_t n_aux
     } else {
         xyz = (R *) b.st_xyz; v = (R *) b.st_vel; rho = (R *) b.st_rho; p = (R *) b.st_p; a = (R *) b.st_acc;
     }
-    k_egress<R><<<nblk(n_state, 256), 256, 0, st>>>(posL, velL, posA, velA, (const Vec4<R> *) b.aux,
-                                                    (const Vec4<R> *) b.pos_u, (const Vec4<R> *) b.vel_u,
-                                                    a ? (const Vec4<R> *) b.acc : nullptr, b.scene_off, n_state,
-                                                    n_aux, n_acc, xyz, v, rho, p, a);
-    return cudaGetLastError();
+    return launch_first(k_egress<R>, nblk(n_state, 256), 256, st, posL, velL, posA, velA, (const Vec4<R> *) b.aux,
+                        (const Vec4<R> *) b.pos_u, (const Vec4<R> *) b.vel_u, a ? (const Vec4<R> *) b.acc : nullptr,
+                        b.scene_off, n_state, n_aux, n_acc, xyz, v, rho, p, a);
 }
 
 template <class R>

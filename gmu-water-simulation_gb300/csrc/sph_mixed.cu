@@ -682,16 +682,14 @@ cudaError_t mixed_egress(const DevBufs &b, uint32_t n_state, uint32_t n_aux, uin
     const Vec4<float> *velA = (const Vec4<float> *) (aux_sorted ? b.vel_s : b.vel_u);
     const Vec4<float> *acc = (const Vec4<float> *) b.acc;
     if (f64)
-        k_egress_mixed<double><<<nblk(n_state, 256), 256, 0, st>>>(
-            posL, loL, velL, posA, velA, (const Vec4<float> *) b.aux, (const Vec4<float> *) b.pos_u,
-            (const Vec4<float> *) b.vel_u, b.st_acc64 ? acc : nullptr, b.scene_off, n_state, n_aux, n_acc, b.st_xyz64,
-            b.st_vel64, b.st_rho64, b.st_p64, b.st_acc64);
-    else
-        k_egress_mixed<float><<<nblk(n_state, 256), 256, 0, st>>>(
-            posL, loL, velL, posA, velA, (const Vec4<float> *) b.aux, (const Vec4<float> *) b.pos_u,
-            (const Vec4<float> *) b.vel_u, b.st_acc ? acc : nullptr, b.scene_off, n_state, n_aux, n_acc, b.st_xyz,
-            b.st_vel, b.st_rho, b.st_p, b.st_acc);
-    return cudaGetLastError();
+        return launch_first(k_egress_mixed<double>, nblk(n_state, 256), 256, st, posL, loL, velL, posA, velA,
+                            (const Vec4<float> *) b.aux, (const Vec4<float> *) b.pos_u, (const Vec4<float> *) b.vel_u,
+                            b.st_acc64 ? acc : nullptr, b.scene_off, n_state, n_aux, n_acc, b.st_xyz64, b.st_vel64,
+                            b.st_rho64, b.st_p64, b.st_acc64);
+    return launch_first(k_egress_mixed<float>, nblk(n_state, 256), 256, st, posL, loL, velL, posA, velA,
+                        (const Vec4<float> *) b.aux, (const Vec4<float> *) b.pos_u, (const Vec4<float> *) b.vel_u,
+                        b.st_acc ? acc : nullptr, b.scene_off, n_state, n_aux, n_acc, b.st_xyz, b.st_vel, b.st_rho,
+                        b.st_p, b.st_acc);
 }
 
 SPH_CHECK_ACCESSOR(check_flags_mixed)
