@@ -321,6 +321,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_forces_mixed(
                     for (int k = 1; k < St::WORDS; k++) m = w == (uint32_t) k ? wr[k] : m;
                 } else {  // beyond the recorded chunks: test the candidates here
                     const uint32_t ce = min(je, cb + 32u);
+                    // 8 loads in flight where crowded windows are walked by a few warps: a fountain of 200,000
+                    // 385 to 375 us; the short rows of cells of h/2 never come here, and keep their registers
+#pragma unroll (RAD == 1 ? 8 : 4)
                     for (uint32_t j = ce; j-- > cb;) {
                         float x, yy, zz;
                         code_delta(gi, __ldg(gpos + j), x, yy, zz);
