@@ -297,9 +297,10 @@ __global__ void __launch_bounds__(kGroupThreads) k_density_group64(
     st4(aux + i, aux_record<double>(rho, rmul(c.k, rsub(rho, c.rho0)), c));
 }
 
-// Bound by the FP64 pipe: about 35 FP64 instructions a pair, most of them the square root and the
-// division, and 2 to sum it. 887 us in the mask form, 272 us here for 50,000 fallen particles; its
-// epilogue with one lane of each group instead of a full warp, and every FP64 cell by division: 365 us.
+// Bound by the FP64 pipe: about 22 FP64 instructions a pair, a third of them the reciprocal root, and 2 to sum
+// it. 50,000 fallen particles: 887 us in the mask form, 272 us here with a square root and a division (365 with
+// its epilogue on one lane of each group instead of a full warp and every FP64 cell by division), 225 us with
+// the reciprocal root.
 template <int G>
 __global__ void __launch_bounds__(kGroupThreads) k_forces_group64(
     const Vec4<double> *__restrict__ pos, const float *__restrict__ posf, const Vec4<double> *__restrict__ vel,

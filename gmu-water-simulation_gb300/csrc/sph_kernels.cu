@@ -431,11 +431,10 @@ __global__ void __launch_bounds__(BLOCK) k_forces_list(
 // 27 cells of size h; RAD = 2 walks 125 cells of size h/2 (42% less volume than 27 h^3).
 
 // Cells of h/2 (RAD 2): short rows, many of them; 75% of the issue slots and 69% of the load path used at
-// 1,000,000 fallen particles, the rest waiting for loads. At 32 registers (8 blocks an SM, a few spills) rather
-// than 48: 4,000,000 fallen 848 to 815 us, 1,000,000 at rest 137 to 133, fallen 223 to 227 alone, but a whole
-// two-step call of the latter beside others 1070 to 1058.
-template <class R, bool REC, int RAD = 1>
-__global__ void __launch_bounds__(256, RAD == 2 ? 8 : 1) k_density_mask(const Vec4<R> *__restrict__ pos, Vec4<R> *__restrict__ aux,
+// 1,000,000 fallen particles, the rest waiting for loads. 229 us with a compare, a select and a shift-or for each
+// candidate's bit, 223 with the funnel shift.
+template <class R, bool REC, int RAD = 1, int MINB = 1>
+__global__ void __launch_bounds__(256, MINB) k_density_mask(const Vec4<R> *__restrict__ pos, Vec4<R> *__restrict__ aux,
                                                       const uint32_t *__restrict__ start,
                                                       const SceneDev *__restrict__ scenes, uint32_t n, Consts<R> c,
                                                       uint32_t *__restrict__ masks, const Vec4<R> *__restrict__ vel,
@@ -1111,6 +1110,12 @@ cudaError_t Launch<R>::rehash(const DevBufs &b, uint32_t n, Consts<R> c, cudaStr
     return cudaGetLastError();
 }
 
+// Particles from which the density pass on cells of h/2 runs at 32 registers and 8 blocks an SM (with a few
+// spills) instead of 48 and 5. Below, the launch is a few waves of blocks and the cap costs more than the warps
+// hide: 1,000,000 fallen 227 instead of 223 us, the 500-step dam break 264 instead of 254 us a step. Beyond,
+// 2,500,000 fallen 520 instead of 535 us, 4,000,000 815 instead of 848, a step of 16,000,000 10.04 instead of 10.33 ms.
+constexpr uint32_t kDensityWide = 1u << 21;
+
 template <class R>
 cudaError_t Launch<R>::density(const DevBufs &b, uint32_t n, Consts<R> c, const Tune &t, bool quads, cudaStream_t st)
 {
@@ -1130,8 +1135,9 @@ cudaError_t Launch<R>::density(const DevBufs &b, uint32_t n, Consts<R> c, const 
                                       b.start, b.scenes, n, c, b.masks, (const Vec4<R> *) b.vel_s, (Vec4<R> *) b.frec);
         if (t.cell_mult == 2) {
             if constexpr (sizeof(R) == 4)
-                return launch_chained(k_density_mask<R, true, 2>, nblk(n, 256), 256, st, pos, aux, b.start, b.scenes,
-                                      n, c, b.masks, (const Vec4<R> *) b.vel_s, (Vec4<R> *) b.frec);
+                return launch_chained(n < kDensityWide ? k_density_mask<R, true, 2> : k_density_mask<R, true, 2, 8>,
+                                      nblk(n, 256), 256, st, pos, aux, b.start, b.scenes, n, c, b.masks,
+                                      (const Vec4<R> *) b.vel_s, (Vec4<R> *) b.frec);
             else
                 return cudaErrorInvalidValue;  // the FP64 form runs on the reference's grid only
         } else {

@@ -79,3 +79,23 @@ def test_download_between_the_passes(sphlib):
         ctx.close()
     for k in out[0]:
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.gpu
+def test_half_cells_density_of_large_scenes(sphlib):
+    """Cells of h/2: a scene in a batch of 2^21 particles (density at 32 registers) has the bits that it has
+    alone, one particle short of that."""
+    n = (1 << 21) - 1
+    box, pos, vel = scene(n, "lattice", 13)
+    out = []
+    for sizes in ([n], [n, 1]):
+        ctx = sphlib.SphContext([box] * len(sizes), sizes, gravity=G981)
+        ctx.set_cell_multiple(2)
+        ctx.set_variant(0, 10)
+        extra = sum(sizes) - n
+        ctx.upload(np.concatenate([pos, pos[:extra]]), np.concatenate([vel, vel[:extra]]), sizes)
+        ctx.step(1)
+        out.append(ctx.download())
+        ctx.close()
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k][:n]), k
