@@ -590,9 +590,9 @@ float elapsed(cudaEvent_t a, cudaEvent_t b)
 // try each in turn. The candidates are four record-reading variants of one kernel (7: no
 // register cap, blocks of 256 threads; 9: 40 registers, blocks of 256; 10 and 11: 40 and 48
 // registers, blocks of 128), whose order depends on how latency-bound the pass is: the
-// collapsing dam break settles on 9 or 10, the dense fountain on 7. Every online_period steps, one step runs with each candidate,
-// timed from the start of its grid pass to the end of its force pass; the fastest is kept
-// until the next trial. A trial step waits for its own end (one host synchronisation per
+// collapsing dam break settles on 9 or 10, the dense fountain on 7. Every online_period steps, one
+// step runs with each candidate, timed from the start of its grid pass to the end of its force
+// pass; the fastest is kept until the next trial. A trial step waits for its own end (one host synchronisation per
 // candidate).
 // The mixed form's candidates are its four launch forms (blocks of 128 or 256 threads, with and
 // without a 48-register cap).
@@ -600,7 +600,14 @@ constexpr int kOnlineCand[kOnlineN] = {7, 9, 10, 11};
 constexpr int kOnlineCandMixed[kOnlineN] = {0, 1, 2, 3};
 static_assert(kOnlineN == kMixedVariants, "every mixed variant is an online candidate");
 
-int online_candidate(const sph_ctx *c, int k) { return is_mixed(c) ? kOnlineCandMixed[k] : kOnlineCand[k]; }
+// Where variant 3 is a group form it takes the first candidate's place: 8,000 particles over a 1,000-step run 30.5
+// us a step, 49 when the tuner could only leave it for the record variants.
+bool group_form(const sph_ctx *c, int m) { return m == 1 && !is_mixed(c) && (is_f64(c) || c->n <= kGroupMax); }
+int online_candidate(const sph_ctx *c, int m, int k)
+{
+    if (is_mixed(c)) return kOnlineCandMixed[k];
+    return k == 0 && group_form(c, m) ? 3 : kOnlineCand[k];
+}
 
 bool online_active(const sph_ctx *c)
 {
@@ -624,13 +631,14 @@ int online_begin_step(sph_ctx *c)
         const int m = c->tune.cell_mult;
         for (int k = 0; k < kOnlineN; k++, c->n_trials++) {
             c->trial_m[c->n_trials] = m;
-            c->trial_v[c->n_trials] = online_candidate(c, k);
+            c->trial_v[c->n_trials] = online_candidate(c, m, k);
         }
         const int other = m == 1 ? 2 : 1;
         if (!c->cell_pinned && cell_mult_allowed(c, other, c->ctot_ref)) {
             c->trial_m[c->n_trials] = other;
             c->trial_v[c->n_trials] = is_mixed(c) ? std::min(c->last_best_v[other], kMixedVariants - 1)
-                                                  : std::max(7, c->last_best_v[other]);
+                                  : group_form(c, other) ? 3
+                                                         : std::max(7, c->last_best_v[other]);
             c->n_trials++;
         }
     }
