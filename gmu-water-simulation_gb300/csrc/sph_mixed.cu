@@ -659,7 +659,9 @@ static cudaError_t mixed_forces_rad(const DevBufs &b, uint32_t n, Consts<float> 
     case 1: return launch_forces_mixed<10, 128, RAD>(b, n, c, mc, record_acc, st);
     case 2: return launch_forces_mixed<1, 256, RAD>(b, n, c, mc, record_acc, st);
     case 3: return launch_forces_mixed<5, 256, RAD>(b, n, c, mc, record_acc, st);
-    default: return launch_forces_mixed<8, 128, RAD>(b, n, c, mc, record_acc, st);
+    // (0 on cells of h/2: as 1. Their shorter rows leave room for it: 4,000,000 fallen 1188 to 1161 us, 1,000,000
+    // 311 to 307, at rest 164 to 162; on cells of h 326 to 334 us fallen, 150 to 145 at rest)
+    default: return launch_forces_mixed<RAD == 2 ? 10 : 8, 128, RAD>(b, n, c, mc, record_acc, st);
     }
 }
 

@@ -200,8 +200,9 @@ int sph_pass_times(sph_ctx *ctx, double ms[5]);
  *            registers (5 and 6 blocks of 256 per SM); 10 and 11 are 9 and 8 launched in
  *            blocks of 128 threads (12 and 10 per SM). SPH_ERR_ARG for other numbers.
  * The mixed form has one density pass (density_variant 0) and force variants 0..3: blocks of
- * 128 threads at up to 64 or 48 registers (0, the default, with several lanes per particle in
- * scenes of up to 32,768 particles on cells of h), blocks of 256 with no cap or 48 registers. On cells
+ * 128 threads at up to 64 or 48 registers (0, the default, at 48 on cells of h/2 and with several
+ * lanes per particle in scenes of up to 32,768 particles on cells of h), blocks of 256 with no cap or
+ * 48 registers. On cells
  * of h/2 (sph_set_cell_multiple) the plain form runs density 0 with force variants 7..11. */
 int sph_set_variant(sph_ctx *ctx, int32_t density_variant, int32_t forces_variant);
 int sph_get_variant(const sph_ctx *ctx, int32_t out[2]);
