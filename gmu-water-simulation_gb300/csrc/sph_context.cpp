@@ -1575,15 +1575,15 @@ int get_grid_ref(sph_ctx *c, uint32_t *cell_of_particle, uint32_t *cell_counts, 
         cmax = std::max<uint64_t>(cmax, (uint64_t) h.res[0] * h.res[1] * h.res[2]);
     }
     const uint64_t nb = cmax / kScanTile + 1;
-    const uint64_t words = nmax + (cmax + 1) + nmax + cmax + nmax + nb + big_words(nmax);
+    const uint64_t words = 2 * ((nmax + 1) / 2) + big_words(nmax) + nmax + (cmax + 1) + nmax + cmax + nb;
     uint32_t *mem = nullptr;
     CK(c, cudaMalloc(&mem, 4 * words));
-    uint32_t *d_cell = mem, *d_start = d_cell + nmax, *d_order = d_start + cmax + 1;
     GridScratch g;
+    g.tmp = mem;  // these two first: aligned
+    g.big = g.tmp + 2 * ((nmax + 1) / 2);
+    uint32_t *d_cell = g.big + big_words(nmax), *d_start = d_cell + nmax, *d_order = d_start + cmax + 1;
     g.count = d_order + nmax;
-    g.tmp = g.count + cmax;
-    g.bsum = g.tmp + nmax;
-    g.big = g.bsum + nb;
+    g.bsum = g.count + cmax;
     uint64_t off = 0, cbase = 0;
     cudaError_t e = cudaSuccess;
     std::vector<uint32_t> cell, start, order;

@@ -53,6 +53,9 @@ __device__ __forceinline__ void chain_wait()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The same without letting the next kernel be scheduled before this one's blocks end.
+__device__ __forceinline__ void chain_wait_last() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <typename... K, typename... A>
 inline cudaError_t launch_chained(void (*kernel)(K...), unsigned grid, unsigned block, cudaStream_t st, A... args)
 {

@@ -60,8 +60,8 @@ struct DevBufs {
     uint32_t *count;       // particles per global cell (hash output; the slot pass counts it back to 0)
     uint32_t *start;       // exclusive scan of count, ncells_total + 1 entries
     uint32_t *bsum;        // particles per kScanTile-cell group (Consts::gsum), ncells / kScanTile + 1 words
-    uint32_t *big;         // allocation-free build only (else null): cells above kBigCell particles, their number
-                           // in word 0, then the cells (big_words(n) words)
+    uint32_t *big;         // allocation-free build only (else null): the lists of crowded cells (big_words(n) words)
+    uint32_t big_room, big_from;  // the n of those lists / kBigCell; particles beyond which a cell is listed
     SceneDev *scenes;
     ObstacleDev *obstacles;
     uint32_t *scene_off;   // first output index of every scene (id-order downloads)
@@ -167,12 +167,17 @@ constexpr int kMaskWordsPerParticle = 36;
 // size (plus one), enough for any tile size, and is sized with it wherever it is allocated.
 constexpr uint32_t kScanTile = 1024;
 
-// In the allocation-free grid build, cells holding more than kBigCell particles are listed by the scan
-// and ordered by a whole block (k_order_cells), in shared memory up to kBigCellMax particles. The
-// list holds its length in word 0 and at most n / kBigCell cells: big_words(n) words.
+// In the allocation-free grid build the scan lists the cells of more than kBigCell particles (or more than
+// a larger number, DevBufs::big_from), each as its first slot and the one behind its last, by what orders them
+// (k_order): up to kWarpCell and up to kSplitCell particles a warp a cell, beyond several warps. Words 0 to 2 hold the
+// three numbers of cells; from word kBigHead on follow room = n / kBigCell entries of two words for the first
+// list from the front and the second from the back (each cell holds more than kBigCell particles, so they
+// cannot meet), then n / kSplitCell entries for the third: big_words(n) words, 8-byte aligned.
 constexpr uint32_t kBigCell = 32;
-constexpr uint32_t kBigCellMax = 4096;
-__host__ __device__ constexpr uint64_t big_words(uint64_t n) { return n / kBigCell + 2; }
+constexpr uint32_t kWarpCell = 128;
+constexpr uint32_t kSplitCell = 512;
+constexpr uint32_t kBigHead = 4;
+__host__ __device__ constexpr uint64_t big_words(uint64_t n) { return kBigHead + 2 * (n / kBigCell + n / kSplitCell + 1); }
 
 // ---- kernel launchers (sph_kernels.cu) --------------------------------------------
 template <class R>
@@ -235,7 +240,7 @@ cudaError_t launch_splat(const DevBufs &b, uint32_t n, int layout_sorted, uint32
                          uint32_t *count, float *depth, cudaStream_t st);
 
 // Working memory of a reference-grid build of n particles and C cells: counts (C words), slot
-// ids (n), group sums (C / kScanTile + 1), crowded cells (big_words(n)).
+// ids (n, 16-byte aligned), group sums (C / kScanTile + 1), crowded cells (big_words(n), 8-byte aligned).
 struct GridScratch {
     uint32_t *count, *tmp, *bsum, *big;
 };

@@ -142,7 +142,7 @@ template <int Q>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const uint32_t *__restrict__ count, uint32_t ncells,
                                                              const uint32_t *__restrict__ gsum,
                                                              uint32_t *__restrict__ start, bool vec,
-                                                             uint32_t *__restrict__ big)
+                                                             uint32_t *__restrict__ big, uint32_t room, uint32_t from)
 {
     chain_wait();
     uint4 c4[Q];
@@ -169,11 +169,17 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const uint32_t *__r
         const uint32_t run = block_exclusive_scan(c.x + c.y + c.z + c.w, total) + off;
         off += total;
         const uint4 st4v = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
-        if (big) {  // cells above kBigCell particles are listed (for the allocation-free build)
-            const uint32_t cv[4] = {c.x, c.y, c.z, c.w};
+        if (big) {  // the crowded cells are listed (for the allocation-free build)
+            const uint32_t cv[4] = {c.x, c.y, c.z, c.w}, sv[4] = {st4v.x, st4v.y, st4v.z, st4v.w};
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                if (cv[k] > kBigCell) big[1 + atomicAdd(big, 1u)] = base + (uint32_t) k;
+            for (int k = 0; k < 4; k++) {
+                if (cv[k] <= from) continue;
+                uint32_t at;
+                if (cv[k] <= kWarpCell) at = atomicAdd(big, 1u);
+                else if (cv[k] <= kSplitCell) at = room - 1 - atomicAdd(big + 1, 1u);
+                else at = room + atomicAdd(big + 2, 1u);
+                reinterpret_cast<uint2 *>(big + kBigHead)[at] = make_uint2(sv[k], sv[k] + cv[k]);
+            }
         }
         if (vec && base + 4 <= ncells) {
             *reinterpret_cast<uint4 *>(start + base) = st4v;
@@ -1082,10 +1088,12 @@ cudaError_t Launch<R>::scan(const DevBufs &b, uint32_t ncells, cudaStream_t st)
     const bool vec = ((reinterpret_cast<uintptr_t>(b.count) | reinterpret_cast<uintptr_t>(b.start)) & 15u) == 0;
     if (ncells >= kScanLargeGrid) {
         const uint32_t nb = (ncells + 4 * SCAN_GROUP - 1) / (4 * SCAN_GROUP);
-        return launch_chained(k_scan_apply<4>, nb, SCAN_THREADS, st, b.count, ncells, b.bsum, b.start, vec, b.big);
+        return launch_chained(k_scan_apply<4>, nb, SCAN_THREADS, st, b.count, ncells, b.bsum, b.start, vec, b.big,
+                              b.big_room, b.big_from);
     }
     const uint32_t nb = (ncells + SCAN_GROUP - 1) / SCAN_GROUP;
-    return launch_chained(k_scan_apply<1>, nb, SCAN_THREADS, st, b.count, ncells, b.bsum, b.start, vec, b.big);
+    return launch_chained(k_scan_apply<1>, nb, SCAN_THREADS, st, b.count, ncells, b.bsum, b.start, vec, b.big,
+                              b.big_room, b.big_from);
 }
 
 template <class R>

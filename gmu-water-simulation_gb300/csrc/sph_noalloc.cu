@@ -19,6 +19,7 @@
 // different streams, or from different host threads) race on it and must not be issued.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 
@@ -33,8 +34,8 @@ constexpr uint32_t kMaxParticles = 1u << 20;
 constexpr uint32_t kMaxCells = 1u << 20;
 constexpr uint32_t kMaxBlocks = kMaxCells / kScanTile + 1;  // group sums of the scan
 constexpr size_t kBigWords = big_words(kMaxParticles);       // crowded-cell list
-// counts | slot ids | group sums | crowded cells, as 32-bit words
-constexpr size_t kScratchWords = (size_t) kMaxCells + kMaxParticles + kMaxBlocks + kBigWords;
+// counts | slot ids | crowded cells | group sums, as 32-bit words
+constexpr size_t kScratchWords = (size_t) kMaxCells + kMaxParticles + kBigWords + kMaxBlocks;
 
 __device__ __align__(256) uint32_t g_grid_scratch[kScratchWords];
 
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(256) k_hash_plain_xyz(const float *__restrict_
                                                         uint32_t *__restrict__ slot, uint32_t *__restrict__ big)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) big[0] = 0;  // the crowded-cell list, for the scan
+    if (i < kBigHead) big[i] = 0;  // the crowded cells' lists, for the scan
     if (i >= n) return;
     const int cx = cell_axis(xyz[3 * i], half.x, inv_h, h_d, res.x);
     const int cy = cell_axis(xyz[3 * i + 1], half.y, inv_h, h_d, res.y);
@@ -94,88 +95,154 @@ __global__ void __launch_bounds__(256) k_group_sums(const uint32_t *__restrict__
     }
 }
 
-// every id to its slot of its cell
+// Every id to its slot of its cell. It lets the next kernel be scheduled only as it ends: k_order's blocks would
+// else be placed beside this kernel's, several on some SMs and none on others, and those that order crowded
+// cells would share an SM (60,000 particles in 18 cells 150 us, so 43).
 __global__ void __launch_bounds__(256) k_slot_ids(const uint32_t *__restrict__ cell, uint32_t n,
                                                   const uint32_t *__restrict__ start,
                                                   const uint32_t *__restrict__ slot, uint32_t *__restrict__ slot_ids)
 {
-    chain_wait();
+    chain_wait_last();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     slot_ids[start[cell[i]] + slot[i]] = i;
 }
 
-// Canonical (cell, id) order: position = cell start + number of same-cell ids below i, counted. A thread a
-// particle: up to kRankByParticle particles, where even a single cell of them all is a few million
-// loads; beyond, k_order_cells.
-constexpr uint32_t kRankByParticle = 65536;
+// Canonical (cell, id) order: position = cell start + number of same-cell ids below i, counted. Cells up to the
+// number of particles from which the scan lists them are ordered by a thread a particle (k_order<false>: it
+// reads two cell starts and the slots of a random cell), or by a thread a cell (k_order<true>: neighbouring
+// threads read and write neighbouring slots), the listed ones by warps and blocks.
+//
+// A thread a cell wants many cells of few particles each: beyond kOrderByCell particles and from a sixth as many
+// cells. Whole builds by cell / by particle: 1,000,003 scattered particles in 800,000 cells 50.7 / 54.2 us, 1,000,000
+// at 5 a cell 46 / 54, but 520,000 38.8 / 37.8, 260,000 31 / 28, 70,000 25 / 22, and 400,000 in a fountain, whose
+// crowded cells lie side by side, 62 / 53.
+constexpr uint32_t kOrderByCell = 524288;
+// Cells are listed beyond kBigCell particles, but in builds of up to kFewLists particles only beyond kWarpCell: there a
+// few crowded cells leave most warps idle either way (a fountain of 60,000 26.2 / 28.5 us with the earlier lists,
+// of 30,000 23 / 26), beyond it the scattered loads of a thread a particle bind (200,000 at 100 a cell 59 / 45 us).
+constexpr uint32_t kFewLists = 65536;
 
-__global__ void __launch_bounds__(256) k_rank_ids(const uint32_t *__restrict__ cell, uint32_t n,
-                                                  const uint32_t *__restrict__ start,
-                                                  const uint32_t *__restrict__ slot_ids, uint32_t *__restrict__ order)
+// One where w < id, else zero, for whole numbers. As floats (exact up to 2^24) it is one full-rate FP32
+// instruction, the saturated difference; the integer compare runs at half the rate and needs a second one.
+__device__ __forceinline__ float below(float w, float id)
 {
-    chain_wait();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t c = cell[i], b = start[c], e = start[c + 1];
-    const uint32_t dst = b + count_rank(slot_ids, b, e, i);
-    if (sph_check(dst < e && e <= n, CHK_SORT)) order[dst] = i;
+    float r;
+    asm("sub.sat.f32 %0, %1, %2;" : "=f"(r) : "f"(id), "f"(w));
+    return r;
+}
+__device__ __forceinline__ uint32_t below(uint32_t w, uint32_t id) { return w < id ? 1u : 0u; }
+constexpr uint32_t kFloatIds = 1u << 24;
+
+// kPart of the ids in the slots [b, e) of a crowded cell, from slot k on, two a thread, against all of them,
+// which the block stages 1,024 at a time. Called by whole blocks.
+constexpr uint32_t kPart = 512;
+template <class T>
+struct alignas(16) Quad {
+    T x, y, z, w;
+};
+template <class T>
+__device__ __forceinline__ void place_part(Quad<T> *stage, const uint32_t *__restrict__ slot_ids, uint32_t b, uint32_t e,
+                                           uint32_t k, uint32_t *__restrict__ order)
+{
+    const uint32_t k0 = k + threadIdx.x, k1 = k0 + 256u;
+    const uint32_t id0 = k0 < e ? slot_ids[k0] : 0u, id1 = k1 < e ? slot_ids[k1] : 0u;
+    const T f0 = (T) id0, f1 = (T) id1, none = (T) 0xffffffffu;
+    T r0 = 0, r1 = 0;
+    for (uint32_t c = b & ~3u; c < e; c += 1024u) {
+        const uint32_t j = c + 4u * threadIdx.x;
+        if (j < e) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(slot_ids + j);
+            stage[threadIdx.x] = {j >= b ? (T) v.x : none, j + 1 >= b && j + 1 < e ? (T) v.y : none,
+                                  j + 2 >= b && j + 2 < e ? (T) v.z : none, j + 3 >= b && j + 3 < e ? (T) v.w : none};
+        }
+        __syncthreads();
+        const uint32_t quads = min(256u, (e - c + 3u) / 4u);
+#pragma unroll 4
+        for (uint32_t q = 0; q < quads; q++) {
+            const Quad<T> w = stage[q];
+            r0 += below(w.x, f0), r0 += below(w.y, f0), r0 += below(w.z, f0), r0 += below(w.w, f0);
+            r1 += below(w.x, f1), r1 += below(w.y, f1), r1 += below(w.z, f1), r1 += below(w.w, f1);
+        }
+        __syncthreads();
+    }
+    const uint32_t d0 = b + (uint32_t) r0, d1 = b + (uint32_t) r1;
+    if (k0 < e && sph_check(d0 < e, CHK_SORT)) order[d0] = id0;
+    if (k1 < e && sph_check(d1 < e, CHK_SORT)) order[d1] = id1;
 }
 
-// The same by cells, a thread a cell, so that neighbouring threads read and write neighbouring slots (a
-// thread a particle reads two cell starts and the slots of a random cell). Cells above kBigCell particles
-// are left to the list: those of up to kBigCellMax sorted by one block each (bitonic, in shared memory),
-// larger ones (thousands of times the rest density) counted by all blocks together. The whole build of
-// scattered particles, with this pass and with k_rank_ids: 65,000 22.6 / 18.2 us, 520,000 34.8 / 32.8,
-// 1,040,000 46.5 / 49.2, and k_rank_ids would need a sort of crowded cells before it (3 us) at such sizes.
-__global__ void __launch_bounds__(256) k_order_cells(const uint32_t *__restrict__ start, uint32_t ncells,
-                                                     const uint32_t *__restrict__ slot_ids,
-                                                     const uint32_t *__restrict__ big, uint32_t n,
-                                                     uint32_t *__restrict__ order)
+// The listed cells: up to kWarpCell particles a warp a cell; up to kSplitCell a block a cell; beyond, the parts of
+// all of them dealt out over all blocks, so that no few cells hold one SM up. The lists are walked with the
+// grid's stride or 32 entries at a time: every block reading every entry, or a grid sized by the cells alone,
+// costs milliseconds. Whole builds, in the order 33, 100, 400, 3,000, 8,000 particles a cell: 1,000,000 72, 84,
+// 97, 399, 703 us; 200,000 36, 45, 55, 113, 181; a fountain of 90,000 32, of 400,000 54; 70,000 in one cell 428.
+template <bool BY_CELL>
+__global__ void __launch_bounds__(256) k_order(const uint32_t *__restrict__ cell, const uint32_t *__restrict__ start,
+                                               uint32_t ncells, const uint32_t *__restrict__ slot_ids,
+                                               const uint32_t *__restrict__ big, uint32_t room, uint32_t from,
+                                               uint32_t n, uint32_t *__restrict__ order)
 {
-    __shared__ uint32_t sk[kBigCellMax];
+    __shared__ Quad<uint32_t> stage[256];
     chain_wait();
-    const uint32_t c = blockIdx.x * 256u + threadIdx.x;
-    if (c < ncells) {
-        const uint32_t b = start[c], e = start[c + 1];
-        if (sph_check(b <= e && e <= n, CHK_SORT) && e - b <= kBigCell)
-            for (uint32_t k = b; k < e; k++) {
-                const uint32_t id = slot_ids[k];
-                uint32_t r = b;
-                for (uint32_t m = b; m < e; m++) r += slot_ids[m] < id ? 1u : 0u;
-                order[r] = id;
-            }
-    }
-    const uint32_t nbig = big[0];
-    for (uint32_t q = 0; q < nbig; q++) {
-        const uint32_t cell = big[1 + q];
-        const uint32_t b = start[cell], e = start[cell + 1], occ = e - b;
-        if (!sph_check(b <= e && e <= n, CHK_SORT)) continue;
-        if (occ > kBigCellMax) {
-            for (uint32_t k = b + c; k < e; k += gridDim.x * 256u)
-                order[b + count_rank(slot_ids, b, e, slot_ids[k])] = slot_ids[k];
-            continue;
-        }
-        if (q % gridDim.x != blockIdx.x) continue;
-        uint32_t P = 2 * kBigCell;
-        while (P < occ) P <<= 1;
-        for (uint32_t t = threadIdx.x; t < P; t += 256) sk[t] = t < occ ? slot_ids[b + t] : 0xffffffffu;
-        __syncthreads();
-        for (uint32_t k = 2; k <= P; k <<= 1) {
-            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                for (uint32_t t = threadIdx.x; t < P / 2; t += 256) {
-                    const uint32_t lo = 2 * j * (t / j) + (t % j), hi = lo + j;  // lo has bit j clear
-                    const uint32_t x = sk[lo], y = sk[hi];
-                    if ((x > y) == ((lo & k) == 0)) {
-                        sk[lo] = y;
-                        sk[hi] = x;
-                    }
+    const uint32_t t = blockIdx.x * 256u + threadIdx.x, lane = threadIdx.x & 31u;
+    const uint2 *const list = reinterpret_cast<const uint2 *>(big + kBigHead);
+    const uint32_t few = big[0], many = big[1], most = big[2];
+    if (BY_CELL) {
+        if (t < ncells) {
+            const uint32_t b = start[t], e = start[t + 1];
+            if (sph_check(b <= e && e <= n, CHK_SORT) && e - b <= from)
+                for (uint32_t k = b; k < e; k++) {
+                    const uint32_t id = slot_ids[k];
+                    uint32_t r = b;
+                    for (uint32_t m = b; m < e; m++) r += slot_ids[m] < id ? 1u : 0u;
+                    order[r] = id;
                 }
-                __syncthreads();
-            }
         }
-        for (uint32_t t = threadIdx.x; t < occ; t += 256) order[b + t] = sk[t];
-        __syncthreads();
+    } else if (t < n) {
+        const uint32_t c = cell[t], b = start[c], e = start[c + 1];
+        if (sph_check(b <= e && e <= n, CHK_SORT) && e - b <= from) {
+            const uint32_t dst = b + count_rank(slot_ids, b, e, t);
+            if (sph_check(dst < e, CHK_SORT)) order[dst] = t;
+        }
+    }
+    auto part = [&](uint32_t b, uint32_t e, uint32_t k) {
+        if (n <= kFloatIds) place_part((Quad<float> *) stage, slot_ids, b, e, k, order);
+        else place_part(stage, slot_ids, b, e, k, order);
+    };
+    // a warp a cell
+    for (uint32_t q = t >> 5; q < few; q += gridDim.x * 8u) {
+        const uint2 be = list[q];
+        if (!sph_check(be.x <= be.y && be.y <= n, CHK_SORT)) continue;
+        for (uint32_t k = be.x + lane; k < be.y; k += 32u) {
+            const uint32_t id = slot_ids[k], dst = be.x + count_rank(slot_ids, be.x, be.y, id);
+            if (sph_check(dst < be.y, CHK_SORT)) order[dst] = id;
+        }
+    }
+    // a block a cell
+    for (uint32_t q = blockIdx.x; q < many; q += gridDim.x) {
+        const uint2 be = list[room - 1 - q];
+        if (!sph_check(be.x <= be.y && be.y <= n, CHK_SORT)) continue;
+        for (uint32_t k = be.x; k < be.y; k += kPart) part(be.x, be.y, k);
+    }
+    // a part a block, the parts of all cells dealt out over all blocks; 32 cells of the list at a time
+    for (uint32_t q0 = 0, turn = blockIdx.x; q0 < most; q0 += 32u) {
+        uint2 be = make_uint2(0, 0);
+        if (q0 + lane < most) be = list[room + q0 + lane];
+        if (!sph_check(be.x <= be.y && be.y <= n, CHK_SORT)) be = make_uint2(0, 0);
+        const uint32_t parts = (be.y - be.x + kPart - 1) / kPart;
+        uint32_t upto = parts;  // of this cell and the ones before it
+#pragma unroll
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, upto, 31);
+        for (; turn < total; turn += gridDim.x) {
+            const int s = __ffs(__ballot_sync(0xffffffffu, upto > turn)) - 1;
+            const uint32_t b = __shfl_sync(0xffffffffu, be.x, s), e = __shfl_sync(0xffffffffu, be.y, s);
+            part(b, e, b + (turn - __shfl_sync(0xffffffffu, upto - parts, s)) * kPart);
+        }
+        turn -= total;
     }
 }
 
@@ -194,6 +261,8 @@ cudaError_t ref_grid_build(const float *xyz, uint32_t n, int3 res, float3 half, 
     b.tmp = g.tmp;
     b.bsum = g.bsum;
     b.big = g.big;
+    b.big_room = n / kBigCell;
+    b.big_from = n > kFewLists ? kBigCell : kWarpCell;
     b.start = out_start;
     // the counts start empty (a previous call, or one that failed, may have left values)
     cudaError_t e = cudaMemsetAsync(b.count, 0, 4 * ncells, st);
@@ -209,11 +278,12 @@ cudaError_t ref_grid_build(const float *xyz, uint32_t n, int3 res, float3 half, 
     if (e == cudaSuccess) e = Launch<float>::scan(b, (uint32_t) ncells, st);  // starts
     if (e == cudaSuccess && n)
         e = launch_chained(k_slot_ids, blocks, 256, st, out_cell, n, out_start, out_order, b.tmp);
-    if (e == cudaSuccess && n)
-        e = n <= kRankByParticle
-                ? launch_chained(k_rank_ids, blocks, 256, st, out_cell, n, out_start, b.tmp, out_order)
-                : launch_chained(k_order_cells, (unsigned) ((ncells + 255) / 256), 256, st, out_start, (uint32_t) ncells,
-                                 b.tmp, b.big, n, out_order);
+    if (e == cudaSuccess && n) {
+        const bool by_cell = n > kOrderByCell && ncells >= n / 6;
+        e = launch_chained(by_cell ? k_order<true> : k_order<false>,
+                           by_cell ? std::max(blocks, (unsigned) ((ncells + 255) / 256)) : blocks, 256, st, out_cell,
+                           out_start, (uint32_t) ncells, b.tmp, b.big, b.big_room, b.big_from, n, out_order);
+    }
     return e;
 }
 
@@ -257,8 +327,8 @@ extern "C" int sph_grid_build_noalloc(const float *xyz, uint32_t n, const float 
     GridScratch g;
     g.count = scratch;
     g.tmp = scratch + (size_t) kMaxCells;
-    g.bsum = scratch + (size_t) kMaxCells + kMaxParticles;
-    g.big = g.bsum + kMaxBlocks;
+    g.big = g.tmp + kMaxParticles;
+    g.bsum = g.big + kBigWords;
     const float3 half = make_float3(box[0] / 2.0f, box[1] / 2.0f, box[2] / 2.0f);
     const cudaError_t e = ref_grid_build(xyz, n, res, half, h, out_cell, out_start, out_order, g, (cudaStream_t) stream);
     return e == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
