@@ -87,17 +87,12 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
     if (cd.x != NONE && sph_check(slot < n, CHK_SORT)) tmp[slot] = cd.y;
     cluster_meet();
     for (uint32_t g = i; g < ncells / kScanTile + 1; g += kSmallParticles) gsum[g] = 0;
-    // canonical rank, and the particle to its place
+    // canonical rank, and the particle to its place (the barrier's acquire lets plain loads see the slots)
     if (i >= n) return;
     place.fetch(i);
     const uint32_t b = __ldcg(start + cd.x), e = __ldcg(start + cd.x + 1);
     if (!sph_check(b <= e && e <= n, CHK_SORT)) return;
-    uint32_t r = b, q = b;
-    for (; q + 8 <= e; q += 8) {
-#pragma unroll
-        for (uint32_t u = 0; u < 8; u++) r += __ldcg(tmp + q + u) < cd.y ? 1u : 0u;
-    }
-    for (; q < e; q++) r += __ldcg(tmp + q) < cd.y ? 1u : 0u;
+    const uint32_t r = b + count_rank(tmp, b, e, cd.y);
     if (sph_check(r < e, CHK_SORT)) place.store(r);
 }
 
