@@ -491,15 +491,20 @@ int run_density(sph_ctx *c)
     return SPH_OK;
 }
 
-// The variant set now, or, where it was changed since the density pass to one that reads what that
-// pass did not write, the variant of that pass: the force records (plain, 4 to 6 write masks alone),
-// the masks (FP64, 3 writes none). All of them give the same bits.
+// What a variant's density pass leaves for the force pass, and what its force pass reads of that: nothing (0 to 2,
+// and the FP64 form's 3), the masks (4 to 6), the masks and the force records (the others).
+int handed_over(const sph_ctx *c, int forces_mode)
+{
+    if (forces_mode <= 2 || (forces_mode == 3 && is_f64(c))) return 0;
+    return forces_mode >= 4 && forces_mode <= 6 ? 1 : 2;
+}
+
+// The variant set now, or, where it was changed since the density pass to one that reads what that pass did not
+// write, the variant of that pass. All of them give the same bits.
 Tune forces_tune(const sph_ctx *c)
 {
     Tune t = c->tune;
-    const bool reads_records = (t.forces_mode == 3 && !is_f64(c)) || (t.forces_mode >= 7 && t.forces_mode <= 11);
-    if (is_f64(c) && c->dense_mode == 3 && t.forces_mode >= 4 && t.forces_mode <= 11) t.forces_mode = 3;
-    else if (reads_records && c->dense_mode >= 4 && c->dense_mode <= 6) t.forces_mode = c->dense_mode;
+    if (handed_over(c, t.forces_mode) > handed_over(c, c->dense_mode)) t.forces_mode = c->dense_mode;
     return t;
 }
 template <class R>
