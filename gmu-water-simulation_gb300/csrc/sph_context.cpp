@@ -606,13 +606,17 @@ constexpr int kOnlineCandMixed[kOnlineN] = {0, 1, 2, 3};
 static_assert(kOnlineN == kMixedVariants, "every mixed variant is an online candidate");
 
 // Where variant 3 is a group form it takes the first candidate's place: 8,000 particles over a 1,000-step run 30.5
-// us a step, 49 when the tuner could only leave it for the record variants.
+// us a step, 49 when the tuner could only leave it for the record variants. In the FP64 form it is the only one: the mask
+// forms take two to seven times as long at every size, and with three trial steps of theirs in a period of 50 a run of
+// 50,000 fallen particles took 347 us a step instead of 302, one of 2,000 at rest 58 instead of 44.
 bool group_form(const sph_ctx *c, int m) { return m == 1 && !is_mixed(c) && (is_f64(c) || c->n <= kGroupMax); }
 int online_candidate(const sph_ctx *c, int m, int k)
 {
     if (is_mixed(c)) return kOnlineCandMixed[k];
     return k == 0 && group_form(c, m) ? 3 : kOnlineCand[k];
 }
+
+int online_candidates(const sph_ctx *c) { return is_f64(c) ? 1 : kOnlineN; }
 
 bool online_active(const sph_ctx *c)
 {
@@ -624,7 +628,7 @@ bool online_active(const sph_ctx *c)
 int set_cell_mult(sph_ctx *c, int m);
 bool cell_mult_allowed(const sph_ctx *c, int m, uint64_t ctot_ref);
 
-// A trial period times the form's four variants on the current cell multiple and, unless the
+// A trial period times the form's variants on the current cell multiple and, unless the
 // multiple was set by the caller, the other multiple once (with the variant its last trials
 // kept): the column's state decides which grid is faster, and it changes over a run.
 int online_begin_step(sph_ctx *c)
@@ -634,7 +638,7 @@ int online_begin_step(sph_ctx *c)
         c->trial = 0;
         c->n_trials = 0;
         const int m = c->tune.cell_mult;
-        for (int k = 0; k < kOnlineN; k++, c->n_trials++) {
+        for (int k = 0; k < online_candidates(c); k++, c->n_trials++) {
             c->trial_m[c->n_trials] = m;
             c->trial_v[c->n_trials] = online_candidate(c, m, k);
         }
