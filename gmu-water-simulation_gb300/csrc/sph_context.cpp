@@ -718,6 +718,8 @@ std::string tune_cache_path()
     return std::string(home && *home ? home : "/tmp") + "/.cache/sph_gb300/tune.txt";
 }
 
+// The key of a choice; kTuneRules ends it since the group forms exist. A key without it is an older library's.
+constexpr const char *kTuneRules = "|v2";
 std::string tune_key(const sph_ctx *c, uint64_t n)
 {
     std::string dev = c->devname;
@@ -726,10 +728,19 @@ std::string tune_key(const sph_ctx *c, uint64_t n)
     return dev + "|p" + std::to_string(c->prm.precision) + "|b" + std::to_string(bucket_of(n));
 }
 
+// Whether an older library's choice is out of date: on cells of h, where the default is a group form now, that
+// library could only choose among the one-thread forms, which are slower there and give the same bits.
+bool tune_outdated(const sph_ctx *c, int fv, int mv)
+{
+    if (mv != 1) return false;
+    return is_mixed(c) ? c->n <= kGroupMax && fv != 0 : group_form(c, 1) && fv != 3;
+}
+
 // cached (density, forces, cell multiple) choice for key, if any; lines are "key d f m" (a line
 // without m is cell multiple 1)
 bool tune_lookup(const sph_ctx *c, const std::string &key, int &dv, int &fv, int &mv)
 {
+    const std::string now = key + kTuneRules;
     const std::string path = tune_cache_path();
     if (access(path.c_str(), R_OK) != 0) return false;  // (every upload asks: cheaper than an open that fails)
     std::ifstream f(path);
@@ -739,8 +750,9 @@ bool tune_lookup(const sph_ctx *c, const std::string &key, int &dv, int &fv, int
         std::istringstream is(line);
         std::string k;
         int d, fo, m = 1;
-        if (!(is >> k >> d >> fo) || k != key) continue;
+        if (!(is >> k >> d >> fo) || (k != key && k != now)) continue;
         if (!(is >> m)) m = 1;
+        if (k == key && tune_outdated(c, fo, m)) continue;
         if (cell_mult_allowed(c, m, c->ctot_ref) && valid_variant(c, d, fo, m)) {
             dv = d;
             fv = fo;
@@ -757,7 +769,7 @@ void tune_store(const std::string &key, int dv, int fv, int mv)
     for (size_t p = path.find('/', 1); p != std::string::npos; p = path.find('/', p + 1))
         mkdir(path.substr(0, p).c_str(), 0755);
     std::ofstream f(path, std::ios::app);
-    if (f) f << key << " " << dv << " " << fv << " " << mv << "\n";
+    if (f) f << key << kTuneRules << " " << dv << " " << fv << " " << mv << "\n";
 }
 
 
