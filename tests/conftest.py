@@ -1,5 +1,6 @@
 import os
 import sys
+import tempfile
 
 import pytest
 
@@ -13,6 +14,8 @@ for p in (ROOT, PKG, os.path.join(ROOT, "tests")):
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (runs on the GB300 box)")
     config.addinivalue_line("markers", "slow: long-running GPU case at full benchmark size")
+    # choices cached by other runs on this machine would change what the tests run on
+    os.environ.setdefault("SPH_TUNE_CACHE", os.path.join(tempfile.mkdtemp(prefix="sph_tune_"), "tune.txt"))
 
 
 @pytest.fixture(scope="session")
