@@ -417,8 +417,12 @@ class SphContext:
 
         cnt = torch.empty((height, width), dtype=torch.int32, device="cuda")
         dep = torch.empty((height, width), dtype=torch.float32, device="cuda")
-        s = torch.cuda.current_stream()
-        self.splat_raw(scene, axis, width, height, cnt.data_ptr(), dep.data_ptr(), s.cuda_stream)
+        # each stream waits for the other, the default stream too (NULL names no consumer to sph_splat): the
+        # images' memory may still be in use here, and they are read here
+        here, ctx = torch.cuda.current_stream(), torch.cuda.ExternalStream(self.stream)
+        ctx.wait_stream(here)
+        self.splat_raw(scene, axis, width, height, cnt.data_ptr(), dep.data_ptr())
+        here.wait_stream(ctx)
         return cnt.cpu().numpy().view(np.uint32), dep.cpu().numpy()
 
     def grid(self):
