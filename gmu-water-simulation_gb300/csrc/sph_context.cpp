@@ -127,15 +127,6 @@ MixConsts make_mix(const sph_params &p)
 }
 size_t r4_bytes(const sph_ctx *c) { return is_f64(c) ? 32 : 16; }
 
-// The hash outputs of a grid of ncells cells cleared: the per-cell counts and their per-group sums
-// (the step's own passes leave both empty between steps).
-int clear_counts(sph_ctx *c, uint64_t ncells)
-{
-    // the group sums lie before the counts in one array: one memset for both
-    CK(c, cudaMemsetAsync(c->b.bsum, 0, (char *) (c->b.count + ncells) - (char *) c->b.bsum, c->stream));
-    return SPH_OK;
-}
-
 template <class R>
 Consts<R> make_consts(const sph_ctx *ctx, int cell_mult)
 {
@@ -238,9 +229,6 @@ void drop_graph(sph_ctx *c)
     c->graph_steps = 0;
 }
 
-// bytes of the group sums of C cells, which precede the counts in their array (both 256-byte aligned)
-size_t sums_bytes(uint64_t C) { return (4 * ((C + kScanTile - 1) / kScanTile + 1) + 255) & ~size_t(255); }
-
 struct PoolItem {
     void **p;
     size_t bytes;
@@ -255,6 +243,20 @@ constexpr size_t kCanaryBytes = 0;
 #endif
 constexpr unsigned char kCanary = 0xA5;
 
+// The hash outputs of a grid of ncells cells cleared: the per-cell counts and their per-group sums
+// (the step's own passes leave both empty between steps).
+int clear_counts(sph_ctx *c, uint64_t ncells)
+{
+    DevBufs &b = c->b;
+    if (kCanaryBytes) {  // a guard region lies between the two
+        CK(c, cudaMemsetAsync(b.bsum, 0, 4 * (ncells / kScanTile + 1), c->stream));
+        CK(c, cudaMemsetAsync(b.count, 0, 4 * ncells, c->stream));
+    } else {  // the counts follow the group sums in the pool: one memset for both
+        CK(c, cudaMemsetAsync(b.bsum, 0, (char *) (b.count + ncells) - (char *) b.bsum, c->stream));
+    }
+    return SPH_OK;
+}
+
 // The sub-arrays of a context's single device allocation (256-byte aligned); returns the
 // total size. Needs only the configuration (no CUDA call), so a create can be refused before
 // any device work and sph_memory_required can answer on the host.
@@ -263,7 +265,6 @@ size_t pool_layout(sph_ctx *c, std::vector<PoolItem> &items)
     const size_t r4 = r4_bytes(c), rs = is_f64(c) ? 8 : 4;
     const bool mixed = is_mixed(c);
     const uint64_t N = c->ncap, C = c->ctot_cap;
-    const size_t sums = sums_bytes(C);
     uint64_t nobs = 0;
     for (auto &h : c->sc) nobs += h.obs.size();
     DevBufs &b = c->b;
@@ -272,7 +273,8 @@ size_t pool_layout(sph_ctx *c, std::vector<PoolItem> &items)
         {&b.pos_s, r4 * N}, {&b.vel_s, r4 * N}, {&b.pos_u, r4 * N}, {&b.vel_u, r4 * N}, {&b.aux, r4 * N},
         {&b.acc, rec ? r4 * N : 0},
         {(void **) &b.cid_u, 8 * N}, {(void **) &b.tmp, 4 * N},
-        {(void **) &b.bsum, sums + 4 * C}, {(void **) &b.start, 4 * (C + 1)},
+        {(void **) &b.bsum, 4 * ((C + kScanTile - 1) / kScanTile + 1)}, {(void **) &b.count, 4 * C},
+        {(void **) &b.start, 4 * (C + 1)},
         {(void **) &b.scenes, sizeof(SceneDev) * c->sc.size()},
         {(void **) &b.obstacles, sizeof(ObstacleDev) * (nobs ? nobs : 1)},
         {(void **) &b.scene_off, 4 * (c->sc.size() + 1)},
@@ -327,7 +329,6 @@ int allocate(sph_ctx *c)
             p += kCanaryBytes;
         }
     }
-    b.count = (uint32_t *) ((char *) b.bsum + sums_bytes(C));
     if (int rc = clear_counts(c, C)) return rc;
     CK(c, cudaMemsetAsync(b.aux, 0, r4 * N, c->stream));
     return SPH_OK;
