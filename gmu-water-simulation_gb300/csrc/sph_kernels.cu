@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(256, MINB) k_density_mask(const Vec4<R> *__res
             }
         }
     }
-    const R rho = rmul(rmul(-acc, c.c_poly6), c.mass);
+    const R rho = rmul(rmul(rsub((R) 0, acc), c.c_poly6), c.mass);  // (+0 for a particle without neighbours or self: NaN)
     const R p = rmul(c.k, rsub(rho, c.rho0));
     const Vec4<R> ar = aux_record<R>(rho, p, c);
     const R q = ar.z, inv = ar.w;
