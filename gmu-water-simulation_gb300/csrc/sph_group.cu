@@ -198,7 +198,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_forces_group(
 // float r^2 of a pair at distance h lies within 4u h^2 + 7.4 u h X + 13.3 u^2 X^2 of h^2, farther pairs'
 // above and nearer pairs' below that. Each coefficient of the margin is more than twice that: a pair
 // beyond it is rejected, a pair inside it accepted, and only the few within it need the exact test. A
-// NaN or an infinity anywhere goes to the exact test.
+// NaN or an infinity anywhere goes to the exact test. Where h^2 is so small that the squares are denormal, the
+// roundings are absolute, at most 2^-150 each: the last term of the margin, 2^-145, is more than three times the ten
+// of them in r^2, h^2 and the margin itself.
 struct FloatTest {
     float x, y, z, limit, sure;
     __device__ __forceinline__ FloatTest(const Vec4<double> &p, const Consts<double> &c)
@@ -206,7 +208,7 @@ struct FloatTest {
     {
         constexpr float u = 5.9604645e-8f;
         const float h = c.h_f, X = fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))) + h;
-        const float margin = 32.0f * u * h * (h + X) + 128.0f * (u * X) * (u * X);
+        const float margin = 32.0f * u * h * (h + X) + 128.0f * (u * X) * (u * X) + 2.2420775e-44f;
         limit = h * h + margin;
         sure = h * h - margin;
         if (!(X < 3.0e38f)) limit = sure = __int_as_float(0x7fffffff);  // NaN: every candidate to the exact test
