@@ -204,9 +204,9 @@ __device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf
 __device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float inv_sqrt(float x) { return rsqrtf(x); }
 // rsqrt rather than 1.0 / sqrt(x): the FP64 force pass is bound by its FP64 instructions, and a correctly rounded
-// root and division are two thirds as many again as the rest of a pair. Its error over (0, h^2] is the smaller
-// one too: at most 0.51 ulp (rms 0.29) against 1.49 (rms 0.45) for the two roundings. One step of 50,000
-// fallen particles, uploaded and read back: 534 to 488 us.
+// root and division are two thirds as many again as the rest of a pair. CUDA documents at most 1 ulp for it; over
+// 4,000,000 sampled arguments in (0, h^2] its largest error was 0.51 ulp (rms 0.29), that of the two roundings 1.49
+// (rms 0.45). One step of 50,000 fallen particles, uploaded and read back: 534 to 488 us.
 __device__ __forceinline__ double inv_sqrt(double x) { return rsqrt(x); }
 // For x that is normal (or zero, infinite, NaN): the hardware's approximation by itself, without the scaling
 // of denormal arguments that rsqrtf surrounds it with; the same value for every normal x.

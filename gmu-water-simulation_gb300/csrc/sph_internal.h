@@ -65,8 +65,10 @@ struct DevBufs {
     SceneDev *scenes;
     ObstacleDev *obstacles;
     uint32_t *scene_off;   // first output index of every scene (id-order downloads)
-    // staging for host transfers (ingest / egress); between a grid pass and its density pass st_xyz also
-    // holds rounded positions (FP64) or quads of positions (plain)
+    // staging for host transfers (ingest / egress). From a grid pass on st_xyz also holds quads of positions up to
+    // the density pass (plain; a transfer between the two overwrites them, sph_ctx::quads says whether they are there)
+    // or rounded positions up to the end of the force pass (FP64; nothing else writes it meanwhile: FP64 transfers
+    // to the caller go through the *64 arrays, transfers from the caller need a completed step)
     float *st_xyz, *st_vel, *st_rho, *st_p, *st_acc;
     double *st_xyz64, *st_vel64, *st_rho64, *st_p64, *st_acc64;
     double *stats;         // per-scene FP64 reductions, 8 doubles each
@@ -135,9 +137,9 @@ struct MixConsts {
 //   forces_mode: 0 = pair terms inside the candidate loop; 1/2 = compacted neighbour list
 //               of 32/64 entries per thread in shared memory; 3..11 = driven by the neighbour
 //               masks that the density pass then writes (density_p is ignored): 3, the default,
-//               in group form (sph_group.cu) for up to kGroupMax particles of the plain form and for
-//               the FP64 form, else as 4; 3/4 one neighbour per iteration without/with a 64-register cap, 5/6 two per
-//               iteration with/without it, 7 as 6 with each neighbour's terms read from one
+//               in group form (sph_group.cu) for up to kGroupMax particles of the plain form and for the
+//               FP64 form, else as 7 below kRecordsCapped particles and as 10 from there on; 4 one neighbour per
+//               iteration, 5/6 two per iteration with/without a 64-register cap, 7 as 6 with each neighbour's terms read from one
 //               packed force record (two 16-byte loads from one 32-byte record), 8 and 9 as
 //               7 at 48 and 40 registers, 10 and 11 as 9 and 8 in blocks of 128 threads
 //   cell_mult : the step grid's cells are h / cell_mult wide (1 or 2); the neighbour passes walk
