@@ -114,13 +114,13 @@ __global__ void __launch_bounds__(256) k_slot_ids(const uint32_t *__restrict__ c
 // threads read and write neighbouring slots), the listed ones by warps and blocks.
 //
 // A thread a cell wants many cells of few particles each: beyond kOrderByCell particles and from a sixth as many
-// cells. Whole builds by cell / by particle: 1,000,003 scattered particles in 800,000 cells 50.7 / 54.2 us, 1,000,000
-// at 5 a cell 46 / 54, but 520,000 38.8 / 37.8, 260,000 31 / 28, 70,000 25 / 22, and 400,000 in a fountain, whose
-// crowded cells lie side by side, 62 / 53.
+// cells. Whole builds by cell / by particle: 1,000,003 scattered particles in 800,000 cells 50.7 / 54.3 us, 1,000,000
+// at 5 a cell 46.5 / 55, but 520,000 38.2 / 37.7, 260,000 30.7 / 27.5, 70,000 24.9 / 21.1, and 400,000 in a fountain,
+// whose crowded cells lie side by side, 62 / 53.
 constexpr uint32_t kOrderByCell = 524288;
 // Cells are listed beyond kBigCell particles, but in builds of up to kFewLists particles only beyond kWarpCell: there a
-// few crowded cells leave most warps idle either way (a fountain of 60,000 26.2 / 28.5 us with the earlier lists,
-// of 30,000 23 / 26), beyond it the scattered loads of a thread a particle bind (200,000 at 100 a cell 59 / 45 us).
+// few crowded cells leave most warps idle either way (with 32 / 128: a fountain of 60,000 27.5 / 24.7 us, of 30,000
+// 25.5 / 22.2), beyond it the scattered loads of a thread a particle bind (200,000 at 100 a cell 38 / 47 us).
 constexpr uint32_t kFewLists = 65536;
 
 // One where w < id, else zero, for whole numbers. As floats (exact up to 2^24) it is one full-rate FP32
@@ -174,8 +174,8 @@ __device__ __forceinline__ void place_part(Quad<T> *stage, const uint32_t *__res
 // The listed cells: up to kWarpCell particles a warp a cell; up to kSplitCell a block a cell; beyond, the parts of
 // all of them dealt out over all blocks, so that no few cells hold one SM up. The lists are walked with the
 // grid's stride or 32 entries at a time: every block reading every entry, or a grid sized by the cells alone,
-// costs milliseconds. Whole builds, in the order 33, 100, 400, 3,000, 8,000 particles a cell: 1,000,000 72, 84,
-// 97, 399, 703 us; 200,000 36, 45, 55, 113, 181; a fountain of 90,000 32, of 400,000 54; 70,000 in one cell 428.
+// costs milliseconds. Whole builds, in the order 33, 100, 400, 3,000, 8,000 particles a cell: 1,000,000 65, 65,
+// 97, 399, 703 us; 200,000 34, 38, 55, 113, 180; a fountain of 90,000 30, of 400,000 53; 70,000 in one cell 428.
 template <bool BY_CELL>
 __global__ void __launch_bounds__(256) k_order(const uint32_t *__restrict__ cell, const uint32_t *__restrict__ start,
                                                uint32_t ncells, const uint32_t *__restrict__ slot_ids,

@@ -223,8 +223,9 @@ int sph_get_cell_multiple(const sph_ctx *ctx);
  * current state (per cell multiple the grid pass once, then both neighbour passes re-run from the
  * same sorted inputs per variant pair), the fastest grid + density + forces is kept, and the
  * choice is written to the cache file (SPH_TUNE_CACHE, else $HOME/.cache/sph_gb300/tune.txt)
- * under the device name, precision and particle-count bucket (floor(log2 n)). sph_upload applies
- * a cached choice for its bucket. The simulation advances by exactly one step; reps = timed
+ * under the device name, precision, particle-count bucket (floor(log2 n)) and the version of the
+ * variant rules. sph_upload applies a cached choice for its bucket (an older library's only where
+ * the default is no group form). The simulation advances by exactly one step; reps = timed
  * repetitions per variant (>= 1). */
 int sph_autotune(sph_ctx *ctx, int32_t reps);
 
@@ -232,10 +233,11 @@ int sph_autotune(sph_ctx *ctx, int32_t reps);
  * break packs ~4x more neighbours per particle after a few hundred steps than at the start,
  * and the fastest variant changes with it). Every `period` steps (sph_step or the pass
  * calls), one real step runs with each of the record-reading force variants 7, 9, 10 and 11
- * (the mixed form: its variants 0..3), timed with events on the context's stream (one host
- * synchronisation per trial step), and the fastest is kept until the next trial. All of them
- * compute the same bits, so the results do not depend on the choice; the cell multiple stays.
- * Applies while the current force variant is mask-driven (3..11, or any mixed variant).
+ * (small plain scenes: 3 in the place of 7; the FP64 form: 3 alone; the mixed form: its variants
+ * 0..3), timed with events on the context's stream (one host synchronisation per trial step), and the
+ * fastest is kept until the next trial. All of them compute the same bits, so the results do not
+ * depend on the choice. One more trial step tries the other cell multiple, unless it was set with
+ * sph_set_cell_multiple. Applies while the current force variant is mask-driven (3..11, or any mixed variant).
  * period 0 turns it off (the default); otherwise period >= 4. Not for all-pairs contexts
  * (SPH_ERR_STATE). */
 int sph_set_online_tuning(sph_ctx *ctx, int32_t period);
@@ -252,7 +254,9 @@ int sph_get_resolution(const sph_ctx *ctx, uint32_t scene, int32_t res[3]);
  * SPH_FLAG_RECORD_ACC. Replaces the readback of CGPUBaseParticleSimulator::integrate
  * (src/CGPUBaseParticleSimulator.cpp:84-91). Plain FP32 positions and velocities alone,
  * into 16-byte-aligned pinned arrays, are written there by one gather kernel over the host
- * link (no staging copy); the call returns when the data is in place either way. */
+ * link (no staging copy); the call returns when the data is in place either way. The kernels at
+ * both ends of a call (upload, download, handoff and export) are launched at a priority above that of
+ * an ordinary stream, so they go ahead of the caller's own waiting blocks on the same GPU. */
 int sph_download(sph_ctx *ctx, float *xyz, float *vel, float *rho, float *p, float *acc);
 /* Same in double, for SPH_F64 contexts. */
 int sph_download_f64(sph_ctx *ctx, double *xyz, double *vel, double *rho, double *p, double *acc);
