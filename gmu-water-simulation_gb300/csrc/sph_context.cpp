@@ -1597,6 +1597,7 @@ namespace {
 int get_grid_ref(sph_ctx *c, uint32_t *cell_of_particle, uint32_t *cell_counts, uint32_t *sorted_ids)
 {
     const uint32_t n = c->n;
+    if (int rc = upload_scene_off(c)) return rc;  // particles may have been appended
     c->quads = false;  // the staging arrays are written now
     // id-ordered float positions of the sorted state (the mixed form's hi part: its hash input)
     DevBufs eb = c->b;
